@@ -50,17 +50,19 @@ def algorithmic_bytes(n1: int, nsys: int = 12) -> dict:
         "k_fft_y_inv": 2 * spec,
         "k_fft_x_inv": spec + (9 + 1 + 9) * 8,
         "k_corr": (9 * 4 + 1) * 8 + 1 + 9 * 2 * 8,
-        # velgrad 9, sg 6, sgt 6, wgtc 1, trialtau 2n, gacumgr 1, crss 2n, sch 5n, C~ 36, S 36 | sg 6, edotp 6, gamdot n, trialtau 2n
-        "k_newton": (9 + 6 + 6 + 1 + 2 * nsys + 1 + 2 * nsys + 5 * nsys + 36 + 36 + 6 + 6 + nsys + 2 * nsys) * 8 + 2,
+        # velgrad 9, sg 6, sgt 6, wgtc 1, trialtau 2n, gacumgr 1, crss 2n, sch 5n, C~, C~^-1 and S 21 each (symmetric)
+        # | sg 6, edotp 6, gamdot n, trialtau 2n
+        "k_newton": (9 + 6 + 6 + 1 + 2 * nsys + 1 + 2 * nsys + 5 * nsys + 3 * 21 + 6 + 6 + nsys + 2 * nsys) * 8 + 2,
     }
 
 
-# Counted FP64 arithmetic of k_newton6p (12 slip systems; a fused multiply-add counts 2, a division
-# 1, the integer power |x|^(n-1) by binary powering 8): one constitutive evaluation (resolved shear,
-# power law, plastic strain rate, residual rho and C~ rho, their norm) 612; one Newton step (the
-# tangent dd, the rows of H, Gauss-Jordan on the 6x6 system, the update and its norm) 1000; one
-# hardening update (Voce increment, the 12 x 12 latent-hardening product, the resistance change) 780.
-NEWTON_FLOPS = {"evaluation": 612, "newton_step": 1000, "hardening_update": 780}
+# Counted FP64 arithmetic of k_newtonv (12 slip systems; a fused multiply-add counts 2, the integer
+# power |x|^(n-1) by binary powering 8): one constitutive evaluation (resolved shears, power law,
+# plastic strain rate, tangent dd, residual rho and C~ rho, their norm) 970; one Newton step (H, its
+# L D L^T factors, the substitutions, the update and its norm) 190; one hardening update (the slip
+# rates once more, Voce increment, the 12 x 12 latent-hardening product, the resistances, their
+# reciprocals and their change) 880.
+NEWTON_FLOPS = {"evaluation": 970, "newton_step": 190, "hardening_update": 880}
 
 
 def fp64_peak_tflops(dev) -> float:
@@ -569,10 +571,9 @@ def main(argv=None) -> int:
                 "per_voxel": {"evaluations": nst["evaluations"] / max(nst["voxels"], 1),
                               "newton_steps": nst["newton_steps"] / max(nst["voxels"], 1),
                               "hardening_updates": nst["hardening_updates"] / max(nst["voxels"], 1)},
-                "active_slot_fraction": nst["evaluations"] / (5.0 * nst["eval_passes"]),
-                "active_slot_fraction_newton": nst["newton_steps"] / (5.0 * max(nst["newton_passes"], 1)),
-                "note": "voxel slots: five six-lane groups per warp; a slot idles while the warp waits for its "
-                        "slowest voxel"}
+                "active_slot_fraction": nst["evaluations"] / (32.0 * nst["eval_passes"]),
+                "active_slot_fraction_newton": nst["newton_steps"] / (32.0 * max(nst["newton_passes"], 1)),
+                "note": "voxel slots: one voxel per lane; a slot idles while the warp waits for its slowest voxel"}
 
     cpu = None
     if not args.no_cpu:

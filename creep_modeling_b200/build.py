@@ -19,7 +19,7 @@ OUT = PKG / "_build"
 LIB = OUT / "libevp_b200.so"
 INCLUDE = PKG.parent / "include"
 
-SOURCES = ["evp_solver.cu", "evp_engine.cu", "evp_control.cu", "evp_kernels.cu", "evp_fft.cu", "evp_green.cu",
+SOURCES = ["evp_solver.cu", "evp_engine.cu", "evp_control.cu", "evp_kernels.cu", "evp_newton.cu", "evp_fft.cu", "evp_green.cu",
            "evp_deck.cpp", "evp_server.cpp"]
 # per-file extra flags: the device-side iteration tail keeps plain multiply-then-add rounding
 EXTRA_FLAGS = {"evp_control.cu": ["-fmad=false"]}

@@ -27,6 +27,17 @@ struct PhaseDev {
     double C[81];
 };
 
+// One phase as the local solve reads it (NS: 12 or 24 systems), staged into shared memory by a
+// straight copy.  Systems beyond the phase's own have n = 1 and gamd0 = 0: they never slip.
+template <int NS>
+struct PhaseV {
+    int nsyst, nmodes, int_exp, kuni;  // kuni: the exponent n - 1 when it is one integer for every system, else -1
+    int nsm[3], pad;
+    double ng[2 * NS];                // gamd0, n of each system
+    double hard[NS * NS];             // rows start on 16 bytes
+    double tau1[3], thet0[3], thet1[3], pad2;
+};
+
 // Offsets (in doubles) of the per-kernel results in the small result buffer.
 enum : int {
     OFF_SGAVG = 0,    // 6   sum wgtc*sg over all voxels
@@ -104,6 +115,7 @@ struct Dev {
     int *err;  // error word: bit 0 singular matrix, bit 1 non-finite Newton result, bit 2 form_G failure,
                // bit 3 a TMA bulk copy that did not complete within its bounded wait
     const PhaseDev *ph;
+    const double* phv;  // the phases as PhaseV<12> (at most 12 systems) or PhaseV<24>
     int nph;
 };
 
@@ -280,8 +292,14 @@ void launch_cell2node(const Dev& d, double tdot, int ideriv, cudaStream_t st);
 
 // Batched equilibrium iteration: the member's per-pass launch shape (its single-solve grid
 // and tile) and the launches over a job table (E, jobs: device arrays).
-void member_jobs_voxel(const Dev& d, int modal, MemberJobs& mj);
+void member_jobs_voxel(const Dev& d, MemberJobs& mj);
 void member_jobs_fft(const Dev& d, const FftPlan1D& pl1, const FftPlan1D& pl2, const FftPlan1D& pl3, int prec, MemberJobs& mj);
+struct NewtonShape {
+    int grid, threads, variant;
+    size_t smem;
+};
+NewtonShape newton_shape(const Dev& d);
+void launch_batched_newton(const BatchLaunch& L, const BatchParams& P, cudaStream_t st);
 void launch_batched_voxel(const BatchLaunch& L, const BatchParams& P, cudaStream_t st);
 void launch_batched_fft(const BatchLaunch& L, const BatchParams& P, cudaStream_t st);
 // the serial tail of one iteration for n solves (evp_control.cu); events[i] = EV_* or a status code

@@ -73,7 +73,7 @@ void Engine::set_members(const std::vector<Member>& m) {
     std::vector<MemberJobs> mj(n);
     for (int i = 0; i < n; i++) {
         std::memset(&mj[i], 0, sizeof(MemberJobs));
-        member_jobs_voxel(m[i].e.d, m[i].modal, mj[i]);
+        member_jobs_voxel(m[i].e.d, mj[i]);
         member_jobs_fft(m[i].e.d, m[i].e.pl1, m[i].e.pl2, m[i].e.pl3, m[i].prec, mj[i]);
     }
     // one launch per pass, spectral precision and kernel variant (and per kBatchChunk members),

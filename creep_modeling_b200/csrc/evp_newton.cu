@@ -1,0 +1,923 @@
+// evp_newton.cu -- the local constitutive solve of every equilibrium iteration.
+//   k_newton    solve_res / plastic_strain_rate / elastic_strain_rate / harden
+//               (various_functions.f90:1142-1491) + the stress sums of calc_velgradavg_corr (1556-1578)
+#include "evp_dev.cuh"
+#include "evp_math.cuh"
+#include "evp_vox.cuh"
+
+#include <cstdlib>
+#include <mutex>
+
+namespace evp {
+
+// ---------------------------------------------------------------- k_newton
+template <int NS>
+__device__ __forceinline__ void body_newton1(const Dev& d, const NewtonParams& p, const VB& vb) {
+    const long long N = d.N;
+    double s[14];
+#pragma unroll
+    for (int c = 0; c < 14; c++) s[c] = 0.0;
+    for (long long v = vb.x * (long long)blockDim.x + threadIdx.x; v < N; v += (long long)vb.nx * blockDim.x) {
+        double lam[6], sg[6], sgt[6], D[6];
+        {
+            double vg[9], vs[9], a[6];
+            ld9(d.velgrad, N, v, vg);
+            sym33(vg, vs);
+            t2_to_b6(vs, D);
+            ld6(d.sg, N, v, a);
+            s6_to_b6(a, lam);
+            ld6(d.sgt, N, v, a);
+            s6_to_b6(a, sgt);
+        }
+#pragma unroll
+        for (int i = 0; i < 6; i++) sg[i] = lam[i];
+        const double w = d.wgtc[v];
+        if (d.gas[v]) {
+            double t[6], res[6], out[6], s6v[6];
+#pragma unroll
+            for (int i = 0; i < 6; i++) t[i] = D[i] + sgt[i] / p.tdot * p.complgas;
+#pragma unroll
+            for (int i = 0; i < 6; i++) {
+                double a = 0.0;
+#pragma unroll
+                for (int j = 0; j < 6; j++) a += d.c066mod[(6 * i + j) * N + v] * t[j];
+                res[i] = lam[i] + a;
+            }
+            if (p.modal) {
+#pragma unroll
+                for (int i = 0; i < 6; i++) {
+                    double a = 0.0;
+#pragma unroll
+                    for (int j = 0; j < 6; j++) a += d.cG[(6 * i + j) * N + v] * lam[j];
+                    res[i] -= a;
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 6; i++) {
+                double a = 0.0;
+#pragma unroll
+                for (int j = 0; j < 6; j++) a += d.cgas[(6 * i + j) * N + v] * res[j];
+                out[i] = a;
+            }
+            b6_to_s6(out, s6v);
+            st6(d.sg, N, v, s6v);
+            double z[6] = {0, 0, 0, 0, 0, 0};
+            st6(d.edotp, N, v, z);
+            for (int q = 0; q < d.nsys; q++) d.gamdot[q * N + v] = 0.0;
+#pragma unroll
+            for (int c = 0; c < 6; c++) s[8 + c] += s6v[c] * w;
+            continue;
+        }
+        const PhaseDev& ph = d.ph[d.phase[v]];
+        double tt[NS][2];
+        double taunrm = 0.0;
+#pragma unroll
+        for (int q = 0; q < NS; q++) {
+            tt[q][0] = (q < d.nsys) ? d.trialtau[(2 * q) * N + v] : 0.0;
+            tt[q][1] = (q < d.nsys) ? d.trialtau[(2 * q + 1) * N + v] : 0.0;
+            taunrm += tt[q][0] * tt[q][0] + tt[q][1] * tt[q][1];
+        }
+        taunrm = sqrt(taunrm);
+        double edotth[6] = {0, 0, 0, 0, 0, 0};
+        if (p.thermo) {
+            double e9[9];
+            ld9(d.eth, N, v, e9);
+            t2_to_b6(e9, edotth);
+        }
+        double sgnorm = 0.0;
+#pragma unroll
+        for (int i = 0; i < 6; i++) sgnorm += sg[i] * sg[i];
+        sgnorm = sqrt(sgnorm);
+        const double tolt = fmax(p.error, p.erroral);
+        double errtau = 2.0 * tolt;
+        double edotp[6], dd[15], gamdot[NS], edot[6], res[6], sgold[6] = {0, 0, 0, 0, 0, 0};
+        double dsgnorm = 0.0, ddgnorm = 0.0;
+        const double gamma0 = d.gacumgr[v];
+        for (int itertau = 0; itertau < 10 && errtau > tolt;) {
+            itertau++;
+            int iterNR = 0;
+            double erral = 2.0 * p.erroral, resoldn = 1.0;
+            while (iterNR < 100 && erral > p.erroral) {
+                iterNR++;
+                int icut = 0;
+                double resn = 2.0 * resoldn;
+                while (resn > resoldn && icut < 10) {
+                    constitutive<NS>(ph, d.sch, N, v, tt, sg, edotp, dd, gamdot);
+                    double ds[6];
+#pragma unroll
+                    for (int i = 0; i < 6; i++) ds[i] = (sg[i] - sgt[i]) / p.tdot;
+#pragma unroll
+                    for (int i = 0; i < 6; i++) {
+                        double a = 0.0;
+#pragma unroll
+                        for (int j = 0; j < 6; j++) a += d.sg66[(6 * i + j) * N + v] * ds[j];
+                        edot[i] = edotp[i] + a;
+                        if (p.thermo) edot[i] = edot[i] + edotth[i];
+                    }
+#pragma unroll
+                    for (int i = 0; i < 6; i++) {
+                        double a = 0.0;
+#pragma unroll
+                        for (int j = 0; j < 6; j++) a += d.c066mod[(6 * i + j) * N + v] * (edot[j] - D[j]);
+                        res[i] = sg[i] - lam[i] + a;
+                    }
+                    if (p.modal) {
+                        double r2[6];
+#pragma unroll
+                        for (int i = 0; i < 6; i++) {
+                            double a = 0.0;
+#pragma unroll
+                            for (int j = 0; j < 6; j++) a += d.cG[(6 * i + j) * N + v] * (sg[j] - lam[j]);
+                            r2[i] = a;
+                        }
+#pragma unroll
+                        for (int i = 0; i < 6; i++) res[i] = res[i] - r2[i];
+                    }
+                    resn = 0.0;
+#pragma unroll
+                    for (int i = 0; i < 6; i++) resn += res[i] * res[i];
+                    resn = sqrt(resn);
+                    if (iterNR == 1) resoldn = resn;
+                    if (resn > resoldn) {
+#pragma unroll
+                        for (int i = 0; i < 6; i++) sg[i] = sgold[i] + (sg[i] - sgold[i]) * 0.5;
+                    }
+                    icut++;
+                }
+                resoldn = resn;
+#pragma unroll
+                for (int i = 0; i < 6; i++) sgold[i] = sg[i];
+                double J[36];
+#pragma unroll
+                for (int i = 0; i < 6; i++) {
+                    double crow[6];
+#pragma unroll
+                    for (int k = 0; k < 6; k++) crow[k] = d.c066mod[(6 * i + k) * N + v];
+#pragma unroll
+                    for (int j = 0; j < 6; j++) {
+                        double a = 0.0;
+#pragma unroll
+                        for (int k = 0; k < 6; k++) a += crow[k] * (dd_at(dd, k, j) + d.sg66[(6 * k + j) * N + v] / p.tdot);
+                        J[6 * i + j] = ((i == j) ? 1.0 : 0.0) + a;
+                        if (p.modal) J[6 * i + j] -= d.cG[(6 * i + j) * N + v];
+                    }
+                }
+                if (solve6(J, res) != 0) set_err(d.err, 1);
+                double a = 0.0, b = 0.0, c = 0.0;
+#pragma unroll
+                for (int i = 0; i < 6; i++) {
+                    sg[i] = sg[i] - res[i];
+                    a += (sg[i] - sgold[i]) * (sg[i] - sgold[i]);
+                    b += (sg[i] - lam[i]) * (sg[i] - lam[i]);
+                    c += (edot[i] - D[i]) * (edot[i] - D[i]);
+                }
+                dsgnorm = b;
+                ddgnorm = c;
+                erral = sqrt(a) / sgnorm;
+            }
+            if (p.iuphard) {
+                double tn[NS][2], g1;
+                harden<NS>(ph, d.crss, N, v, gamdot, gamma0, p.tdot, tn, g1);
+                double e2 = 0.0;
+#pragma unroll
+                for (int q = 0; q < NS; q++) {
+                    e2 += (tt[q][0] - tn[q][0]) * (tt[q][0] - tn[q][0]) + (tt[q][1] - tn[q][1]) * (tt[q][1] - tn[q][1]);
+                    tt[q][0] = tn[q][0];
+                    tt[q][1] = tn[q][1];
+                }
+                errtau = sqrt(e2) / taunrm;
+            } else {
+                errtau = 0.0;
+            }
+        }
+        double s6v[6], e6v[6];
+        b6_to_s6(sg, s6v);
+        b6_to_s6(edotp, e6v);
+        st6(d.sg, N, v, s6v);
+        st6(d.edotp, N, v, e6v);
+#pragma unroll
+        for (int q = 0; q < NS; q++)
+            if (q < d.nsys) {
+                d.gamdot[q * N + v] = gamdot[q];
+                d.trialtau[(2 * q) * N + v] = tt[q][0];
+                d.trialtau[(2 * q + 1) * N + v] = tt[q][1];
+            }
+        if (!(dsgnorm == dsgnorm) || !(ddgnorm == ddgnorm)) set_err(d.err, 2);
+        s[0] += dsgnorm * w;
+        s[1] += ddgnorm * w;
+#pragma unroll
+        for (int c = 0; c < 6; c++) {
+            s[2 + c] += w * s6v[c];
+            s[8 + c] += s6v[c] * w;
+        }
+    }
+    reduce_store<14, 0>(s, nullptr, d.partials, d.red + OFF_NEWTON, d.counters + CNT_NEWTON, vb);
+}
+template <int NS>
+__global__ void __launch_bounds__(kNewtonBlock, 2) k_newton(Dev d, NewtonParams p) { body_newton1<NS>(d, p, hw_vb()); }
+// ---------------------------------------------------------------- k_newtonv: one voxel per thread, operators on chip
+// The local solve with one thread per voxel and everything an evaluation reads kept in the
+// block's shared memory, one column per thread (entry i of thread t at [i * blockDim + t], so
+// every access of a warp is conflict free).  With dedot = dd + S / dt the Jacobian of solve_res is
+//   J = I - C~ G + C~ (S / dt + dd) = C~ H,   H = B + S / dt + dd,   B = C~^-1 - G,
+// where G = Gamma~r is the modified augmented Lagrangian's operator (zero without --modal 1;
+// k_prologue_modal leaves C~ G in cG and subtracts G from the stored C~^-1), C~ (c066mod) and S
+// (sg66) are symmetric positive definite, G is symmetric and dd is positive semi-definite.  So
+// the Newton step J^-1 res equals H^-1 rho with rho = C~^-1 res formed directly,
+//   rho = H0 sg + edotp - q',  H0 = B + S / dt,  q' = B lam + (S / dt) sgt + D - eth,
+// and res = C~ rho gives the residual norm that drives the step halving.  H is factored as
+// L D L^T in its 21 entries; a pivot that is not positive (G can only cause that with --modal 1)
+// sends the voxel to the pivoted elimination of the general system.
+// The resistances are used as reciprocals, formed where they change (at the start and at each
+// hardening update, 1.2 per voxel) instead of at each evaluation (3 per voxel); the resistances
+// themselves go to their output array at each update and are read back for the change's norm.
+//
+// What bounds it: latency (global loads of the batch, FP64 chains) at 8 warps per SM: 255 registers
+// a thread and the 840 B column both allow 256 threads per SM with 12 systems, 128 with 24; the
+// systems of an evaluation give each warp independent work, which replaces occupancy.  Against six
+// lanes per voxel, which exchanged every vector between lanes (243 M warp instructions per launch
+// at 64^3, now 64 M), a launch takes 238 us instead of 621 (64^3, 12 systems, n = 20, 3.0
+// evaluations per voxel; 0.50 GB of DRAM traffic, FP64 pipe 28 % busy), 174 instead of 347 (40^3,
+// 24 systems), 35 instead of 105 (32^3, --modal 1), and the same 30 at 16^3, where each SM has one
+// warp and its chain is all there is.  32 voxels of a warp wait for the slowest: 84 % of the slots
+// work.  Measured without gain at 64^3: L2 prefetch of the next batch (290 -> 322 us: two batches of
+// 51 kB per warp do not fit the L2), its asynchronous copies issued before this batch's closing sums
+// (240 -> 243), 12 systems per step (242 -> 324: spills), C~ loaded ahead of the systems (268).
+constexpr int kMaxPhaseSmem = 4;
+// column entries of a thread: Schmid vectors, 1 / resistance (forward, backward), H0 (packed lower triangle)
+template <int NS>
+struct ColV {
+    static constexpr int sch = 0, itau = 5 * NS, h0 = 7 * NS, n = 7 * NS + 21;
+};
+template <int NS>
+__host__ __device__ constexpr int newtonv_threads_per_sm() { return NS <= 12 ? 256 : 128; }
+__host__ __device__ constexpr int tri(int i, int j) { return i >= j ? i * (i + 1) / 2 + j : j * (j + 1) / 2 + i; }
+
+// Loads and stores of fields that the kernel writes, ordered among themselves and known to be global
+// memory (the compiler would otherwise order every shared-memory access around them).
+__device__ __forceinline__ double ld_rw(const double* p) {
+    double x;
+    asm volatile("ld.global.f64 %0, [%1];" : "=d"(x) : "l"(p));
+    return x;
+}
+__device__ __forceinline__ void st_rw(double* p, double x) { asm volatile("st.global.f64 [%0], %1;" ::"l"(p), "d"(x)); }
+
+// the general system by pivoted elimination (rare: see above)
+__device__ __noinline__ int solve_general6(const double* h21, double* b6) {
+    double J[36], b[6];
+#pragma unroll
+    for (int i = 0; i < 6; i++) {
+        b[i] = b6[i];
+#pragma unroll
+        for (int j = 0; j < 6; j++) J[6 * i + j] = h21[tri(i, j)];
+    }
+    const int info = solve6(J, b);
+#pragma unroll
+    for (int i = 0; i < 6; i++) b6[i] = b[i];
+    return info;
+}
+
+// x = H^-1 b in place (H packed, symmetric); returns nonzero when H is singular
+__device__ __forceinline__ int solve_sym6(double (&h)[21], double (&b)[6]) {
+    double a[21], y[6], inv[6];
+    bool spd = true;
+#pragma unroll
+    for (int i = 0; i < 21; i++) a[i] = h[i];
+#pragma unroll
+    for (int i = 0; i < 6; i++) y[i] = b[i];
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+        spd = spd && a[tri(k, k)] > 0.0;
+        inv[k] = rcp_nr(a[tri(k, k)]);
+#pragma unroll
+        for (int i = k + 1; i < 6; i++) {
+            const double l = a[tri(i, k)] * inv[k];
+#pragma unroll
+            for (int j = k + 1; j <= i; j++) a[tri(i, j)] -= l * a[tri(j, k)];
+            y[i] -= l * y[k];
+        }
+    }
+    if (!spd) {
+        double hh[21], bb[6];
+#pragma unroll
+        for (int i = 0; i < 21; i++) hh[i] = h[i];
+#pragma unroll
+        for (int i = 0; i < 6; i++) bb[i] = b[i];
+        const int info = solve_general6(hh, bb);
+#pragma unroll
+        for (int i = 0; i < 6; i++) b[i] = bb[i];
+        return info;
+    }
+    // a(i, k) below the diagonal still holds l_ik d_k
+#pragma unroll
+    for (int i = 5; i >= 0; i--) {
+        double s = y[i];
+#pragma unroll
+        for (int j = i + 1; j < 6; j++) s -= a[tri(j, i)] * b[j];
+        b[i] = s * inv[i];
+    }
+    return 0;
+}
+// y = A x of a packed symmetric A
+__device__ __forceinline__ void sym6_mv(const double (&A)[21], const double (&x)[6], double (&y)[6]) {
+#pragma unroll
+    for (int i = 0; i < 6; i++) {
+        double t = 0.0;
+#pragma unroll
+        for (int j = 0; j < 6; j++) t += A[tri(i, j)] * x[j];
+        y[i] = t;
+    }
+}
+// the upper triangle of a 6x6 operator's planes
+__device__ __forceinline__ void ld_sym6(const double* __restrict__ A, long long N, long long v, double (&a)[21]) {
+#pragma unroll
+    for (int i = 0; i < 6; i++)
+#pragma unroll
+        for (int j = 0; j <= i; j++) a[tri(i, j)] = __ldg(A + (6 * j + i) * N + v);
+}
+template <int M>
+__device__ __forceinline__ void ldg_n(const double* __restrict__ a, long long N, long long v, double* o) {
+#pragma unroll
+    for (int c = 0; c < M; c++) o[c] = __ldg(a + c * N + v);
+}
+__device__ __forceinline__ void cp_async8(double* dst, const double* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+
+// dummy gas voxel: closed-form stress update (various_functions.f90:1165-1185)
+__device__ __forceinline__ void gas_voxel(const Dev& d, const NewtonParams& p, long long v, double (&s6v)[6]) {
+    const long long N = d.N;
+    double lam[6], t[6], a[6], res[6], out[6], vg[9], vs[9];
+    ld9(d.velgrad, N, v, vg);
+    sym33(vg, vs);
+    t2_to_b6(vs, t);
+    ld6(d.sgt, N, v, a);
+    s6_to_b6(a, out);
+#pragma unroll
+    for (int i = 0; i < 6; i++) t[i] = t[i] + out[i] / p.tdot * p.complgas;
+    ld6(d.sg, N, v, a);
+    s6_to_b6(a, lam);
+    for (int i = 0; i < 6; i++) {
+        double x = 0.0;
+        for (int j = 0; j < 6; j++) x += d.c066mod[(6 * i + j) * N + v] * t[j];
+        res[i] = lam[i] + x;
+    }
+    if (p.modal) {
+        for (int i = 0; i < 6; i++) {
+            double x = 0.0;
+            for (int j = 0; j < 6; j++) x += d.cG[(6 * i + j) * N + v] * lam[j];
+            res[i] -= x;
+        }
+    }
+    for (int i = 0; i < 6; i++) {
+        double x = 0.0;
+        for (int j = 0; j < 6; j++) x += d.cgas[(6 * i + j) * N + v] * res[j];
+        out[i] = x;
+    }
+    b6_to_s6(out, s6v);
+    st6(d.sg, N, v, s6v);
+#pragma unroll
+    for (int c = 0; c < 6; c++) d.edotp[c * N + v] = 0.0;
+    for (int q = 0; q < d.nsys; q++) d.gamdot[q * N + v] = 0.0;
+}
+
+// Sums of eight values over the warp by halving exchanges (nine shuffles of a double): lanes
+// 4 q .. 4 q + 3 end with the sum of value sum8_field(lane).
+__device__ __forceinline__ int sum8_field(int lane) { return ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1); }
+__device__ __forceinline__ double warp_sum8(double (&x)[8], int lane) {
+#pragma unroll
+    for (int h = 4; h >= 1; h /= 2) {
+        const bool up = lane & (4 * h);
+#pragma unroll
+        for (int f = 0; f < h; f++) {
+            const double send = up ? x[f] : x[f + h], keep = up ? x[f + h] : x[f];
+            x[f] = keep + __shfl_xor_sync(0xffffffffu, send, 4 * h);
+        }
+    }
+    double y = x[0];
+    y += __shfl_xor_sync(0xffffffffu, y, 2);
+    y += __shfl_xor_sync(0xffffffffu, y, 1);
+    return y;
+}
+
+// Every warp of the block has put its 14 sums into sh -> one partial per block -> the last block
+// folds them in block order; a block of few warps folds its fields together so that their loads
+// overlap.
+constexpr int kNewtonSums = 14;
+__device__ __forceinline__ void reduce_newton(const double (*sh)[kNewtonSums], double* partials, double* out, unsigned int* counter,
+                                              const VB& vb) {
+    constexpr int NF = kNewtonSums;
+    __shared__ bool last;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+    __syncthreads();
+    if (threadIdx.x < NF) {
+        double x = sh[0][threadIdx.x];
+        for (int w = 1; w < nw; w++) x += sh[w][threadIdx.x];
+        partials[(size_t)threadIdx.x * vb.nx + vb.x] = x;
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = (atomicAdd(counter, 1u) == (unsigned)vb.nx - 1u);
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    if (nw >= 4) {
+        for (int f = warp; f < NF; f += nw) {
+            const double x = fold_sum(partials, vb.nx, f, lane);
+            if (lane == 0) out[f] = x;
+        }
+    } else if (warp == 0) {
+        double s[NF];
+#pragma unroll
+        for (int f = 0; f < NF; f++) s[f] = 0.0;
+        for (int b = lane; b < vb.nx; b += 32)
+#pragma unroll
+            for (int f = 0; f < NF; f++) s[f] += __ldcg(partials + (size_t)f * vb.nx + b);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int f = 0; f < NF; f++) s[f] += __shfl_down_sync(0xffffffffu, s[f], o);
+        if (lane == 0)
+#pragma unroll
+            for (int f = 0; f < NF; f++) out[f] = s[f];
+    }
+    if (threadIdx.x == 0) *counter = 0;
+}
+
+// Resolved shears over resistance rs and powers |rs|^(n-1) of G systems (Schmid vectors cs,
+// reciprocal resistances ci, (gamd0, n) pairs ng), each step on all of them so that their chains overlap.
+template <int G>
+__device__ __forceinline__ void slip_powers(const double* cs, const double* ci, const double* ng, int kuni,
+                                            const double (&sg)[6], double (&rs)[G], double (&pw)[G]) {
+#pragma unroll
+    for (int q = 0; q < G; q++) {
+        double x = cs[5 * q * 32] * sg[0];
+#pragma unroll
+        for (int c = 1; c < 5; c++) x += cs[(5 * q + c) * 32] * sg[c];
+        rs[q] = x * ci[2 * q * 32 + (x < 0.0 ? 32 : 0)];
+    }
+    if (kuni >= 0) {  // one integer exponent: binary powering of the systems together
+        double b[G];
+#pragma unroll
+        for (int q = 0; q < G; q++) {
+            b[q] = fabs(rs[q]);
+            pw[q] = (kuni & 1) ? b[q] : 1.0;
+        }
+        for (int k = kuni >> 1; k; k >>= 1) {
+#pragma unroll
+            for (int q = 0; q < G; q++) b[q] *= b[q];
+            if (k & 1)
+#pragma unroll
+                for (int q = 0; q < G; q++) pw[q] *= b[q];
+        }
+    } else {
+#pragma unroll
+        for (int q = 0; q < G; q++) pw[q] = pow(fabs(rs[q]), ng[2 * q + 1] - 1.0);
+    }
+}
+
+template <int NS>
+__device__ __forceinline__ void body_newtonv(const Dev& d, const NewtonParams& p, const VB& vb) {
+    using Col = ColV<NS>;
+    extern __shared__ __align__(16) double dyn_smem[];
+    PhaseV<NS>* const sph = reinterpret_cast<PhaseV<NS>*>(dyn_smem);
+    const int nph = d.nph;  // at most kMaxPhaseSmem (newton_kernel)
+    for (int e = threadIdx.x; e < nph * (int)(sizeof(PhaseV<NS>) / 8); e += blockDim.x) dyn_smem[e] = d.phv[e];
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    double* const col = reinterpret_cast<double*>(sph + nph) + (threadIdx.x >> 5) * (Col::n * 32) + lane;
+    const long long N = d.N;
+    const int qlast = 2 * d.nsys - 1, slast = 5 * d.nsys - 1;
+    constexpr int kG = 6;  // systems per step of an evaluation (of 12 the kernel spills)
+    const double tolt = fmax(p.error, p.erroral), idt = 1.0 / p.tdot;
+    const bool stats = d.nstats != nullptr;
+    unsigned c_pass = 0, c_eval = 0, c_nr = 0, c_tau = 0, c_vox = 0, c_npass = 0;
+    double mine = 0.0, mineg = 0.0;  // running sum sum8_field(lane) of this warp: dsg and ddg norms, stress (solid; gas)
+    const long long stride = (long long)vb.nx * blockDim.x;
+    for (long long v0 = (long long)vb.x * blockDim.x + (threadIdx.x & ~31); v0 < N; v0 += stride) {  // warp-uniform
+        const long long v = v0 + lane;
+        double sums[8], gsum[8];
+#pragma unroll
+        for (int c = 0; c < 8; c++) {
+            sums[c] = 0.0;
+            gsum[c] = 0.0;
+        }
+        if (v < N) {
+            const bool gas = __ldg(d.gas + v);
+            const PhaseV<NS>& ph = sph[__ldg(d.phase + v)];
+            // The batch's inputs are all in flight together: the resistances, B and the Schmid vectors go
+            // to the column by asynchronous copies (no registers wait for them), the rest to registers.
+            double l6[6], t6[6], vg[9], e9[9], sm[21], a[9];
+            {
+                const double* q = d.trialtau + v;
+#pragma unroll
+                for (int i = 0; i < 2 * NS; i++) {
+                    cp_async8(col + (Col::itau + i) * 32, q);
+                    q += i < qlast ? N : 0;
+                }
+                q = d.c066inv + v;
+#pragma unroll
+                for (int i = 0; i < 6; i++)
+#pragma unroll
+                    for (int j = 0; j <= i; j++) cp_async8(col + (Col::h0 + tri(i, j)) * 32, q + (6 * j + i) * N);
+                q = d.sch + v;
+#pragma unroll 10
+                for (int i = 0; i < 5 * NS; i++) {
+                    cp_async8(col + (Col::sch + i) * 32, q);
+                    q += i < slast ? N : 0;
+                }
+            }
+            ld_sym6(d.sg66, N, v, sm);
+#pragma unroll
+            for (int c = 0; c < 6; c++) l6[c] = ld_rw(d.sg + c * N + v);
+            ldg_n<6>(d.sgt, N, v, t6);
+            ldg_n<9>(d.velgrad, N, v, vg);
+            if (p.thermo) ldg_n<9>(d.eth, N, v, e9);
+            const double w = __ldg(d.wgtc + v);
+            double s6v[6];
+            if (gas) {
+                asm volatile("cp.async.wait_all;" ::: "memory");
+                gas_voxel(d, p, v, s6v);
+#pragma unroll
+                for (int c = 0; c < 6; c++) gsum[2 + c] = s6v[c] * w;
+            } else {
+                const int nsyst = ph.nsyst;
+                double sg[6], qp[6], taun = 0.0;
+                {
+                    double sgt[6];
+                    s6_to_b6(l6, sg);
+                    s6_to_b6(t6, sgt);
+                    sym33(vg, a);
+                    t2_to_b6(a, qp);
+                    if (p.thermo) {
+                        t2_to_b6(e9, a);
+#pragma unroll
+                        for (int i = 0; i < 6; i++) qp[i] = qp[i] - a[i];
+                    }
+                    asm volatile("cp.async.wait_all;" ::: "memory");
+#pragma unroll
+                    for (int i = 0; i < 6; i++)
+#pragma unroll
+                        for (int j = 0; j <= i; j++) {
+                            const double bi = col[(Col::h0 + tri(i, j)) * 32], si = sm[tri(i, j)] * idt;
+                            col[(Col::h0 + tri(i, j)) * 32] = bi + si;
+                            qp[i] += bi * sg[j] + si * sgt[j];
+                            if (j != i) qp[j] += bi * sg[i] + si * sgt[i];
+                        }
+#pragma unroll
+                    for (int q = 0; q < 2 * NS; q++) {
+                        const double t = q <= qlast ? col[(Col::itau + q) * 32] : 0.0, i = rcp_nr(t);
+                        taun += t * t;
+                        col[(Col::itau + q) * 32] = q < 2 * nsyst ? i : 0.0;
+                    }
+                    for (int i = 5 * nsyst; i < 5 * NS; i++) col[(Col::sch + i) * 32] = 0.0;
+                }
+                taun = sqrt(taun);
+                double sgnorm2 = 0.0;
+#pragma unroll
+                for (int i = 0; i < 6; i++) sgnorm2 += sg[i] * sg[i];
+                const double sgnorm = sqrt(sgnorm2);
+                const double errlim2 = (p.erroral * sgnorm) * (p.erroral * sgnorm);
+                double sgold[6] = {0, 0, 0, 0, 0, 0}, ep[5] = {0, 0, 0, 0, 0};
+                bool halved = false;  // the last evaluation's stress is in edotp, not in sgold
+                double errtau = 2.0 * tolt;
+                c_vox++;
+                for (int itertau = 0; itertau < 10 && errtau > tolt; itertau++) {
+                    double resold2 = 1.0;
+                    bool more = true;
+                    c_tau++;
+                    for (int iterNR = 0; iterNR < 100 && more; iterNR++) {
+                        // residual norms and the Newton correction are compared as squares (no square
+                        // roots on the chain): res2 = |res|^2, and the loop runs while |dsg|^2 > (erroral |sg_in|)^2
+                        double res2 = 4.0 * resold2, rho[6], dd[15];
+                        for (int icut = 0; icut < 10 && res2 > resold2; icut++) {
+                            if (stats) {
+                                c_eval++;
+                                if (lane == __ffs(__activemask()) - 1) c_pass++;
+                            }
+                            // plastic_strain_rate and its derivative: resolved shears, powers and sums of
+                            // kG systems at a time, each step on all of them so that their chains overlap
+#pragma unroll
+                            for (int c = 0; c < 5; c++) ep[c] = 0.0;
+#pragma unroll
+                            for (int c = 0; c < 15; c++) dd[c] = 0.0;
+#pragma unroll 1
+                            for (int s0 = 0; s0 < NS; s0 += kG) {
+                                const double* const cs = col + (Col::sch + 5 * s0) * 32;
+                                const double* const ci = col + (Col::itau + 2 * s0) * 32;
+                                double rs[kG], pw[kG];
+                                slip_powers<kG>(cs, ci, &ph.ng[2 * s0], ph.kuni, sg, rs, pw);
+#pragma unroll
+                                for (int q = 0; q < kG; q++) {
+                                    const double2 ng = *reinterpret_cast<const double2*>(&ph.ng[2 * (s0 + q)]);
+                                    const double dum = ng.x * pw[q], g = rs[q] * dum;
+                                    const double r1 = ng.y * dum * ci[2 * q * 32 + (rs[q] < 0.0 ? 32 : 0)];
+                                    double sc[5];
+#pragma unroll
+                                    for (int c = 0; c < 5; c++) sc[c] = cs[(5 * q + c) * 32];
+                                    int e = 0;
+#pragma unroll
+                                    for (int jj = 0; jj < 5; jj++) {
+                                        ep[jj] += sc[jj] * g;
+                                        const double t = sc[jj] * r1;
+#pragma unroll
+                                        for (int ii = 0; ii <= jj; ii++) dd[e++] += sc[ii] * t;
+                                    }
+                                }
+                            }
+#pragma unroll
+                            for (int i = 0; i < 6; i++) rho[i] = (i < 5 ? ep[i < 5 ? i : 0] : 0.0) - qp[i];
+#pragma unroll
+                            for (int i = 0; i < 6; i++)
+#pragma unroll
+                                for (int j = 0; j <= i; j++) {
+                                    const double h = col[(Col::h0 + tri(i, j)) * 32];
+                                    rho[i] += h * sg[j];
+                                    if (j != i) rho[j] += h * sg[i];
+                                }
+                            double rn[6], cm[21];
+                            ld_sym6(d.c066mod, N, v, cm);
+                            sym6_mv(cm, rho, rn);
+                            res2 = (rn[0] * rn[0] + rn[1] * rn[1]) + (rn[2] * rn[2] + rn[3] * rn[3]) + (rn[4] * rn[4] + rn[5] * rn[5]);
+                            if (iterNR == 0) resold2 = res2;
+                            halved = false;
+                            if (res2 > resold2) {
+                                if (icut == 9) {
+                                    halved = true;
+#pragma unroll
+                                    for (int i = 0; i < 6; i++) st_rw(d.edotp + i * N + v, sg[i]);
+                                }
+#pragma unroll
+                                for (int i = 0; i < 6; i++) sg[i] = sgold[i] + (sg[i] - sgold[i]) * 0.5;
+                            }
+                        }
+                        resold2 = res2;
+                        if (stats) {
+                            c_nr++;
+                            if (lane == __ffs(__activemask()) - 1) c_npass++;
+                        }
+                        double h[21], dsg2 = 0.0;
+#pragma unroll
+                        for (int i = 0; i < 6; i++)
+#pragma unroll
+                            for (int j = 0; j <= i; j++)
+                                h[tri(i, j)] = col[(Col::h0 + tri(i, j)) * 32] + (i < 5 ? dd[i < 5 ? tri(i, j) : 0] : 0.0);
+                        if (solve_sym6(h, rho) != 0) set_err(d.err, 1);
+#pragma unroll
+                        for (int i = 0; i < 6; i++) {
+                            sgold[i] = sg[i];
+                            sg[i] = sg[i] - rho[i];
+                            dsg2 += (sg[i] - sgold[i]) * (sg[i] - sgold[i]);
+                        }
+                        more = sgnorm > 0.0 ? dsg2 > errlim2 : dsg2 > 0.0;
+                    }
+                    // the slip rates at the last evaluation's stress, formed again (a third of an evaluation)
+                    // instead of kept in registers or written and read back at each evaluation
+                    double gd[NS], dg = 0.0;
+                    {
+                        double se[6], *out = d.gamdot + v;
+#pragma unroll
+                        for (int i = 0; i < 6; i++) se[i] = sgold[i];
+                        if (halved)
+#pragma unroll
+                            for (int i = 0; i < 6; i++) se[i] = ld_rw(d.edotp + i * N + v);
+#pragma unroll
+                        for (int s0 = 0; s0 < NS; s0 += kG) {
+                            double rs[kG], pw[kG];
+                            slip_powers<kG>(col + (Col::sch + 5 * s0) * 32, col + (Col::itau + 2 * s0) * 32, &ph.ng[2 * s0], ph.kuni, se,
+                                            rs, pw);
+#pragma unroll
+                            for (int q = 0; q < kG; q++) {
+                                const double g = rs[q] * (ph.ng[2 * (s0 + q)] * pw[q]);
+                                gd[s0 + q] = fabs(g);
+                                dg += fabs(g);
+                                if (2 * (s0 + q) < qlast) st_rw(out, g);
+                                out += N;
+                            }
+                        }
+                    }
+                    if (!p.iuphard) break;
+                    // harden (various_functions.f90:1439-1491).  The new resistances go to their output array;
+                    // the old ones, for the norm of the change, are the column's reciprocals inverted.
+                    double e2 = 0.0, fm[3];
+                    const double gamma0 = __ldg(d.gacumgr + v);
+                    const double deltgam = dg * p.tdot, gamma1 = gamma0 + deltgam;
+#pragma unroll
+                    for (int m = 0; m < 3; m++) {  // the Voce factor of each mode
+                        fm[m] = 0.0;
+                        if (m < ph.nmodes) {
+                            const double tau1 = ph.tau1[m], thet0 = ph.thet0[m], thet1 = ph.thet1[m];
+                            const double fact = fabs(thet0 / tau1);
+                            const double exp0 = exp(-fact * gamma0), exp1 = exp(-fact * gamma1);
+                            const double voce = deltgam * thet1 + tau1 * (exp0 - exp1) + thet1 * (gamma0 * exp0 - gamma1 * exp1);
+                            fm[m] = voce * p.tdot / deltgam;
+                        }
+                    }
+                    const int m1 = ph.nsm[0], m2 = m1 + ph.nsm[1];
+#pragma unroll 1
+                    for (int s0 = 0; s0 < NS; s0 += 12) {
+                        // every load before the first store: the compiler keeps shared-memory loads behind
+                        // shared-memory stores, which would run the twelve systems one after the other
+                        double cr[24], dtau[12], *out = d.trialtau + 2 * s0 * N + v;
+                        double* const ci = col + (Col::itau + 2 * s0) * 32;
+                        const double* qc = d.crss + (long long)min(2 * s0, qlast) * N + v;
+#pragma unroll
+                        for (int i = 0; i < 24; i++) {
+                            cr[i] = __ldg(qc);
+                            qc += 2 * s0 + i < qlast ? N : 0;
+                        }
+#pragma unroll
+                        for (int q = 0; q < 12; q++) dtau[q] = 0.0;
+#pragma unroll
+                        for (int js = 0; js < NS; js += 2)
+#pragma unroll
+                            for (int q = 0; q < 12; q++) {
+                                const double2 hh = *reinterpret_cast<const double2*>(&ph.hard[(s0 + q) * NS + js]);
+                                dtau[q] += hh.x * gd[js] + hh.y * gd[js + 1];
+                            }
+#pragma unroll
+                        for (int q = 0; q < 12; q++) {
+                            const int s = s0 + q;
+                            const bool own = s < nsyst;
+                            const double x = dtau[q] * (s < m1 ? fm[0] : (s < m2 ? fm[1] : fm[2]));
+                            // systems beyond the phase's own get zero resistance, as harden leaves them
+                            const double n0 = own ? cr[2 * q] + x : 0.0, n1 = own ? cr[2 * q + 1] + x : 0.0;
+                            const double i0 = rcp_nr(n0), i1 = rcp_nr(n1), t0 = rcp_nr(ci[2 * q * 32]), t1 = rcp_nr(ci[(2 * q + 1) * 32]);
+                            const double d0 = own ? t0 - n0 : 0.0, d1 = own ? t1 - n1 : 0.0;
+                            e2 += d0 * d0 + d1 * d1;
+                            ci[2 * q * 32] = own ? i0 : 0.0;
+                            ci[(2 * q + 1) * 32] = own ? i1 : 0.0;
+                            if (2 * s < qlast) {
+                                st_rw(out, n0);
+                                st_rw(out + N, n1);
+                            }
+                            out += 2 * N;
+                        }
+                    }
+                    errtau = sqrt(e2) / taun;
+                }
+                // |sg - lam|^2 at the final stress; |edot - D|^2 at the last evaluation, with
+                // edot = edotp + S (sg - sgt) / dt + eth as elastic_strain_rate forms it
+                double x6[6], e6[6], D[6], e6v[6], dsg = 0.0, ddg = 0.0;
+                ld_sym6(d.sg66, N, v, sm);
+                ldg_n<6>(d.sgt, N, v, t6);
+                ldg_n<9>(d.velgrad, N, v, vg);
+                if (p.thermo) ldg_n<9>(d.eth, N, v, e9);
+#pragma unroll
+                for (int c = 0; c < 6; c++) l6[c] = ld_rw(d.sg + c * N + v);
+                if (halved)
+#pragma unroll
+                    for (int i = 0; i < 6; i++) sgold[i] = ld_rw(d.edotp + i * N + v);
+                s6_to_b6(t6, x6);
+#pragma unroll
+                for (int i = 0; i < 6; i++) x6[i] = (sgold[i] - x6[i]) * idt;
+                sym6_mv(sm, x6, e6);
+                sym33(vg, a);
+                t2_to_b6(a, D);
+                if (p.thermo) t2_to_b6(e9, a);
+                s6_to_b6(l6, x6);
+#pragma unroll
+                for (int i = 0; i < 6; i++) {
+                    double x = (i < 5 ? ep[i < 5 ? i : 0] : 0.0) + e6[i];
+                    if (p.thermo) x = x + a[i];
+                    ddg += (x - D[i]) * (x - D[i]);
+                    dsg += (sg[i] - x6[i]) * (sg[i] - x6[i]);
+                }
+                if (!(dsg == dsg) || !(ddg == ddg)) set_err(d.err, 2);
+                b6_to_s6(sg, s6v);
+#pragma unroll
+                for (int i = 0; i < 6; i++) e6[i] = i < 5 ? ep[i < 5 ? i : 0] : 0.0;
+                b6_to_s6(e6, e6v);
+#pragma unroll
+                for (int c = 0; c < 6; c++) {
+                    st_rw(d.sg + c * N + v, s6v[c]);
+                    st_rw(d.edotp + c * N + v, e6v[c]);
+                    sums[2 + c] = w * s6v[c];
+                }
+                sums[0] = dsg * w;
+                sums[1] = ddg * w;
+            }
+        }
+        __syncwarp();
+        mine += warp_sum8(sums, lane);
+        if (d.cgas) mineg += warp_sum8(gsum, lane);
+    }
+    if (stats) {
+        unsigned c[6] = {c_pass, c_eval, c_nr, c_tau, c_vox, c_npass};
+#pragma unroll
+        for (int i = 0; i < 6; i++) {
+            const unsigned x = __reduce_add_sync(0xffffffffu, c[i]);
+            if (lane == 0) atomicAdd(d.nstats + i, (unsigned long long)x);
+        }
+    }
+    // dsg and ddg norms, the solid's stress sum and the whole cell's
+    __shared__ double sh[8][kNewtonSums];
+    if ((lane & 3) == 0) {
+        const int f = sum8_field(lane);
+        sh[threadIdx.x >> 5][f] = mine;
+        if (f >= 2) sh[threadIdx.x >> 5][f + 6] = mine + mineg;
+    }
+    reduce_newton(sh, d.partials, d.red + OFF_NEWTON, d.counters + CNT_NEWTON, vb);
+}
+template <int NS>
+__global__ void __launch_bounds__(newtonv_threads_per_sm<NS>(), 1) k_newtonv(Dev d, NewtonParams p) { body_newtonv<NS>(d, p, hw_vb()); }
+
+// The local-solve kernel of a solve: 0/1 k_newtonv<12/24> (at most kMaxPhaseSmem phases, whose
+// tables fit beside the columns), 6/7 k_newton<12/24>, which reads every operator from memory
+// (more phases, and EVP_NEWTON_ONE_THREAD=1 for comparison).
+static int newton_kernel(const Dev& d) {
+    static const bool one_thread = [] {
+        const char* e = getenv("EVP_NEWTON_ONE_THREAD");
+        return e && e[0] == '1';
+    }();
+    const int big = d.nsys > 12 ? 1 : 0;
+    return (one_thread || d.nph > kMaxPhaseSmem ? 6 : 0) + big;
+}
+// Block size of k_newtonv: as many threads as an SM holds (one block per SM, the fewest partial
+// sums to fold) unless that leaves SMs without a block; then halved until every SM has one, down
+// to one warp.
+static int newton_threads(const Dev& d, int kernel) {
+    if (kernel >= 6) return kNewtonBlock;
+    int t = kernel == 0 ? newtonv_threads_per_sm<12>() : newtonv_threads_per_sm<24>();
+    while (t > 32 && (d.N + t - 1) / t < 148) t /= 2;
+    return t;
+}
+static int newton_grid(const Dev& d, int kernel) {
+    const long long t = newton_threads(d, kernel), g = (d.N + t - 1) / t;
+    if (kernel >= 6) return (int)(g < 148LL * 16 ? g : 148LL * 16);
+    // one wave, every warp taking every (blocks x warps)-th batch of 32 voxels
+    const long long wave = 148LL * ((kernel == 0 ? newtonv_threads_per_sm<12>() : newtonv_threads_per_sm<24>()) / t);
+    return (int)(g < wave ? g : wave);
+}
+static size_t newton_smem(const Dev& d, int kernel) {
+    const size_t t = newton_threads(d, kernel);
+    switch (kernel) {
+        case 0: return d.nph * sizeof(PhaseV<12>) + sizeof(double) * ColV<12>::n * t;
+        case 1: return d.nph * sizeof(PhaseV<24>) + sizeof(double) * ColV<24>::n * t;
+        default: return 0;
+    }
+}
+template <int V>
+constexpr int kb_newton_bound() { return V >= 6 ? kNewtonBlock : (V == 0 ? newtonv_threads_per_sm<12>() : newtonv_threads_per_sm<24>()); }
+template <int V>
+__global__ void __launch_bounds__(kb_newton_bound<V>(), V >= 6 ? 2 : 1) kb_newton(const __grid_constant__ BatchParams P);
+static void newton_configure() {
+    static std::once_flag once;
+    std::call_once(once, [] {
+        const int lim = 222 * 1024;
+        cudaFuncSetAttribute(k_newtonv<12>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+        cudaFuncSetAttribute(k_newtonv<24>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+        cudaFuncSetAttribute(kb_newton<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+        cudaFuncSetAttribute(kb_newton<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+    });
+}
+
+void launch_newton(const Dev& d, const NewtonParams& p, cudaStream_t st) {
+    newton_configure();
+    const int k = newton_kernel(d), grid = newton_grid(d, k), thr = newton_threads(d, k);
+    const size_t sm = newton_smem(d, k);
+    switch (k) {
+        case 0: k_newtonv<12><<<grid, thr, sm, st>>>(d, p); break;
+        case 1: k_newtonv<24><<<grid, thr, sm, st>>>(d, p); break;
+        case 6: k_newton<12><<<grid, thr, 0, st>>>(d, p); break;
+        default: k_newton<24><<<grid, thr, 0, st>>>(d, p); break;
+    }
+}
+
+template <int V>
+__global__ void __launch_bounds__(kb_newton_bound<V>(), V >= 6 ? 2 : 1) kb_newton(const __grid_constant__ BatchParams P) {
+    __shared__ NewtonParams ps;
+    __shared__ int go;
+    const Job& jb = batch_job(P);
+    const BatchSolve& m = P.E[jb.solve];
+    if (threadIdx.x == 0) {
+        go = m.ctl->active;
+        ps = m.ctl->newton;
+    }
+    __syncthreads();
+    if (!go) return;
+    const NewtonParams p = ps;  // in registers, as a single-solve launch's parameter
+    const VB vb = job_vb(jb);
+    if constexpr (V == 0) body_newtonv<12>(m.d, p, vb);
+    else if constexpr (V == 1) body_newtonv<24>(m.d, p, vb);
+    else if constexpr (V == 6) body_newton1<12>(m.d, p, vb);
+    else body_newton1<24>(m.d, p, vb);
+}
+
+// Launch shape of a solve's local solve.  Members of one block size share a batched launch:
+// variant = kernel + 8 * (block size / 32).
+NewtonShape newton_shape(const Dev& d) {
+    newton_configure();
+    const int k = newton_kernel(d), t = newton_threads(d, k);
+    return NewtonShape{newton_grid(d, k), t, k + 8 * (t / 32), newton_smem(d, k)};
+}
+void launch_batched_newton(const BatchLaunch& L, const BatchParams& P, cudaStream_t st) {
+    switch (L.variant & 7) {
+        case 0: kb_newton<0><<<L.blocks, L.threads, L.smem, st>>>(P); break;
+        case 1: kb_newton<1><<<L.blocks, L.threads, L.smem, st>>>(P); break;
+        case 6: kb_newton<6><<<L.blocks, L.threads, L.smem, st>>>(P); break;
+        default: kb_newton<7><<<L.blocks, L.threads, L.smem, st>>>(P); break;
+    }
+}
+
+}  // namespace evp

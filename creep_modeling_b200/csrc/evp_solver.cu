@@ -250,6 +250,32 @@ public:
         h2d += (long long)bytes;
     }
 
+    // the local solve's phase tables, padded to NS systems
+    template <int NS>
+    const double* upload_phases(const std::vector<PhaseDev>& ph) {
+        std::vector<PhaseV<NS>> t(ph.size());
+        for (size_t p = 0; p < ph.size(); p++) {
+            const PhaseDev& g = ph[p];
+            PhaseV<NS>& v = t[p];
+            std::memset(&v, 0, sizeof(v));
+            v.nsyst = g.nsyst; v.nmodes = g.nmodes; v.int_exp = g.int_exp;
+            v.kuni = g.int_exp && g.nsyst > 0 ? (int)(g.nrs[0] - 1.0) : -1;
+            for (int m = 0; m < 3; m++) {
+                v.nsm[m] = g.nsm[m]; v.tau1[m] = g.tau1[m]; v.thet0[m] = g.thet0[m]; v.thet1[m] = g.thet1[m];
+            }
+            for (int i = 0; i < NS; i++) {
+                const bool own = i < g.nsyst;
+                v.ng[2 * i] = own ? g.gamd0[i] : 0.0;
+                v.ng[2 * i + 1] = own ? g.nrs[i] : 1.0;
+                if (own && g.nrs[i] != g.nrs[0]) v.kuni = -1;
+                for (int j = 0; own && j < g.nsyst; j++) v.hard[i * NS + j] = g.hard[i * kMaxSysDev + j];
+            }
+        }
+        double* dst = dalloc<double>(t.size() * sizeof(PhaseV<NS>) / sizeof(double));
+        h2d_copy(dst, t.data(), t.size() * sizeof(PhaseV<NS>));
+        return dst;
+    }
+
     void sync() { CK(cudaStreamSynchronize(st)); }
     // the result buffer and the error word to the host: queued (fetch_red_async), then read after
     // the stream is synchronised (check_red); fetch_red does both
@@ -456,6 +482,7 @@ public:
         PhaseDev* dph = dalloc<PhaseDev>(dk.nph);
         h2d_copy(dph, ph.data(), dk.nph * sizeof(PhaseDev));
         d.ph = dph;
+        d.phv = d.nsys <= 12 ? upload_phases<12>(ph) : upload_phases<24>(ph);
         d.nph = dk.nph;
     }
 

@@ -1,0 +1,209 @@
+// evp_vox.cuh -- device helpers shared by the per-voxel kernels: block reductions, field loads and
+// stores, the power law and the constitutive law (evp_kernels.cu, evp_newton.cu).
+#pragma once
+#include "evp_dev.cuh"
+#include "evp_math.cuh"
+
+namespace evp {
+
+constexpr int kBlock = 256;
+constexpr int kNewtonBlock = 128;
+constexpr int kC0Block = 64;
+
+// ---------------------------------------------------------------- reductions
+// NS sums then NM maxima per thread -> one partial per block (stored field-major,
+// partials[f * nblocks + block], in the body's block coordinates) -> the last block to finish folds them: one
+// warp per field, lane l adding blocks l, l + 32, ... in order, then a fixed
+// shuffle tree, so the result does not depend on timing (fold_sum, in evp_dev.cuh, for the
+// sums; fold_max for the maxima).
+__device__ __forceinline__ double fold_max(const double* partials, int nblk, int f, int lane) {
+    const double* q = partials + (size_t)f * nblk;
+    double s = -EVP_HUGE;
+    int b = lane;
+    for (; b + 7 * 32 < nblk; b += 8 * 32) {
+        double x[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) x[i] = __ldcg(q + b + 32 * i);
+#pragma unroll
+        for (int i = 0; i < 8; i++) s = fmax(s, x[i]);
+    }
+    for (; b < nblk; b += 32) s = fmax(s, __ldcg(q + b));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s = fmax(s, __shfl_down_sync(0xffffffffu, s, o));
+    return s;  // in lane 0
+}
+
+template <int NS, int NM>
+__device__ void reduce_store(const double* sums, const double* maxs, double* partials, double* out, unsigned int* counter,
+                             const VB& vb) {
+    constexpr int NF = NS + NM;
+    __shared__ double sh[NF][32];
+    __shared__ bool last;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+#pragma unroll
+    for (int f = 0; f < NF; f++) {
+        double x = (f < NS) ? sums[f] : maxs[f - NS];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            double y = __shfl_down_sync(0xffffffffu, x, o);
+            x = (f < NS) ? x + y : fmax(x, y);
+        }
+        if (lane == 0) sh[f][warp] = x;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        for (int f = 0; f < NF; f++) {
+            double x = (lane < nw) ? sh[f][lane] : ((f < NS) ? 0.0 : -EVP_HUGE);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                double y = __shfl_down_sync(0xffffffffu, x, o);
+                x = (f < NS) ? x + y : fmax(x, y);
+            }
+            if (lane == 0) partials[(size_t)f * vb.nx + vb.x] = x;
+        }
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = (atomicAdd(counter, 1u) == (unsigned)vb.nx - 1u);
+    __syncthreads();
+    if (last) {
+        __threadfence();
+        for (int f = warp; f < NF; f += nw) {
+            const double x = (f < NS) ? fold_sum(partials, vb.nx, f, lane) : fold_max(partials, vb.nx, f, lane);
+            if (lane == 0) out[f] = x;
+        }
+        if (threadIdx.x == 0) *counter = 0;
+    }
+}
+
+__device__ __forceinline__ void set_err(int* err, int bit) { atomicOr(err, bit); }
+
+__device__ __forceinline__ void ld9(const double* __restrict__ a, long long N, long long v, double* o) {
+#pragma unroll
+    for (int c = 0; c < 9; c++) o[c] = a[c * N + v];
+}
+__device__ __forceinline__ void st9(double* __restrict__ a, long long N, long long v, const double* o) {
+#pragma unroll
+    for (int c = 0; c < 9; c++) a[c * N + v] = o[c];
+}
+__device__ __forceinline__ void ld6(const double* __restrict__ a, long long N, long long v, double* o) {
+#pragma unroll
+    for (int c = 0; c < 6; c++) o[c] = a[c * N + v];
+}
+__device__ __forceinline__ void st6(double* __restrict__ a, long long N, long long v, const double* o) {
+#pragma unroll
+    for (int c = 0; c < 6; c++) a[c * N + v] = o[c];
+}
+__device__ __forceinline__ void eye9(double* a) {
+#pragma unroll
+    for (int c = 0; c < 9; c++) a[c] = (c % 4 == 0) ? 1.0 : 0.0;
+}
+
+// 1 / x by Newton-Raphson from the hardware's approximation (rcp.approx.ftz.f64, 20 bits: two steps
+// of y += y (1 - x y) reach FP64 rounding).  Branch free, so that independent reciprocals overlap:
+// the compiler's division tests for its slow path one quotient after the other.  For normal x whose
+// reciprocal is normal; 1 / 0 gives NaN.
+__device__ __forceinline__ double rcp_nr(double x) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    y = fma(y, fma(-x, y, 1.0), y);
+    return fma(y, fma(-x, y, 1.0), y);
+}
+
+// |x|^e for the power law: integer exponents by binary powering, else pow().
+__device__ __forceinline__ double powabs(double x, double e, int int_exp) {
+    double a = fabs(x);
+    if (int_exp) {
+        int k = (int)e;
+        double r = 1.0, b = a;
+        while (k) {
+            if (k & 1) r *= b;
+            b *= b;
+            k >>= 1;
+        }
+        return r;
+    }
+    return pow(a, e);
+}
+
+// ---------------------------------------------------------------- local constitutive solve
+// plastic_strain_rate (various_functions.f90:1367-1419) + elastic_strain_rate (1422-1436)
+template <int NS>
+__device__ __forceinline__ void constitutive(const PhaseDev& ph, const double* __restrict__ sch, long long N, long long v,
+                                             const double (&tt)[NS][2], const double (&sg)[6], double (&edotp)[6],
+                                             double (&dd)[15], double (&gamdot)[NS]) {
+#pragma unroll
+    for (int i = 0; i < 6; i++) edotp[i] = 0.0;
+#pragma unroll
+    for (int i = 0; i < 15; i++) dd[i] = 0.0;
+#pragma unroll
+    for (int is = 0; is < NS; is++) {
+        if (is < ph.nsyst) {
+            double sc[5];
+#pragma unroll
+            for (int c = 0; c < 5; c++) sc[c] = sch[(is * 5 + c) * N + v];
+            double rss = sc[0] * sg[0] + sc[1] * sg[1] + sc[2] * sg[2] + sc[3] * sg[3] + sc[4] * sg[4];
+            const double tau = (rss - 0.0 < 0.0) ? tt[is][1] : tt[is][0];  // kin(is) == 0
+            rss = (rss - 0.0) / tau;
+            const double dum = ph.gamd0[is] * powabs(rss, ph.nrs[is] - 1.0, ph.int_exp);
+            const double rss1 = ph.nrs[is] * dum / tau;
+            const double rss2 = rss * dum;
+            gamdot[is] = rss2;
+            int q = 0;
+#pragma unroll
+            for (int jj = 0; jj < 5; jj++) {
+                edotp[jj] = edotp[jj] + sc[jj] * rss2;
+#pragma unroll
+                for (int ii = 0; ii <= jj; ii++) dd[q++] += sc[ii] * sc[jj] * rss1;
+            }
+        } else {
+            gamdot[is] = 0.0;
+        }
+    }
+}
+// x[i] for a run-time i in 0..5 without a local-memory array
+__device__ __forceinline__ double sel6(const double (&x)[6], int i) {
+    double y = x[0];
+#pragma unroll
+    for (int c = 1; c < 6; c++) y = (i == c) ? x[c] : y;
+    return y;
+}
+__device__ __forceinline__ double dd_at(const double (&dd)[15], int i, int j) {
+    if (i > 4 || j > 4) return 0.0;
+    int a = i < j ? i : j, b = i < j ? j : i;
+    return dd[b * (b + 1) / 2 + a];
+}
+
+// harden (various_functions.f90:1439-1491)
+template <int NS>
+__device__ __forceinline__ void harden(const PhaseDev& ph, const double* __restrict__ crss, long long N, long long v,
+                                       const double (&gamdot)[NS], double gamma0, double tdot, double (&tau)[NS][2], double& gamma1) {
+    double deltgam = 0.0;
+#pragma unroll
+    for (int is = 0; is < NS; is++)
+        if (is < ph.nsyst) deltgam = deltgam + fabs(gamdot[is]) * tdot;
+    gamma1 = gamma0 + deltgam;
+#pragma unroll
+    for (int is = 0; is < NS; is++) { tau[is][0] = 0.0; tau[is][1] = 0.0; }
+    int is = 0;
+    for (int mode = 0; mode < ph.nmodes; mode++) {
+        const double tau1 = ph.tau1[mode], thet0 = ph.thet0[mode], thet1 = ph.thet1[mode];
+        const double fact = fabs(thet0 / tau1);
+        const double exp0 = exp(-fact * gamma0), exp1 = exp(-fact * gamma1);
+        const double voce = deltgam * thet1 + tau1 * (exp0 - exp1) + thet1 * (gamma0 * exp0 - gamma1 * exp1);
+        for (int ism = 0; ism < ph.nsm[mode]; ism++, is++) {
+            double dtau = 0.;
+#pragma unroll
+            for (int js = 0; js < NS; js++)
+                if (js < ph.nsyst) dtau = dtau + ph.hard[is * kMaxSysDev + js] * fabs(gamdot[js]);
+#pragma unroll
+            for (int q = 0; q < NS; q++)
+                if (q == is) {
+                    tau[q][0] = crss[(2 * q) * N + v] + dtau * voce * tdot / deltgam;
+                    tau[q][1] = crss[(2 * q + 1) * N + v] + dtau * voce * tdot / deltgam;
+                }
+        }
+    }
+}
+
+}  // namespace evp

@@ -95,9 +95,9 @@ int evp_kernel_times(evp_solve* s, char* names, long long* launches, double* ms,
 long long evp_kernel_launches(evp_solve* s);
 /* Activity counters of the local Newton kernel since open (EVP_PROFILE solves only; no
  * counterpart in the reference): out6[0] warp passes of the evaluation loop, [1] voxel
- * evaluations done in those passes (five voxel groups per warp), [2] Newton steps, [3]
+ * evaluations done in those passes (32 voxels per warp), [2] Newton steps, [3]
  * hardening updates, [4] voxels solved, [5] warp passes of the Newton-step loop.
- * [1] / (5 [0]) is the fraction of voxel slots that did useful work. */
+ * [1] / (32 [0]) is the fraction of voxel slots that did useful work. */
 int evp_newton_stats(evp_solve* s, long long* out6);
 
 /* Operator-level entry: applies the periodic Green operator of a homogeneous
