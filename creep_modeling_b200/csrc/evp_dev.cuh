@@ -290,6 +290,11 @@ void launch_c0(const Dev& d, double tdot, double tdotref, cudaStream_t st);
 void launch_kinematic(const Dev& d, double tdot_step, cudaStream_t st);
 void launch_cell2node(const Dev& d, double tdot, int ideriv, cudaStream_t st);
 
+// out[v * nout + c] = in[map[c] * N + v0 + v] for v in [0, nv): a field's planes as one record per voxel
+constexpr int kMaxInterleave = 5 * kMaxSysDev;
+void launch_interleave(const Dev& d, const double* in, const int* map, int nout, long long v0, long long nv, double* out,
+                       cudaStream_t st);
+
 // Batched equilibrium iteration: the member's per-pass launch shape (its single-solve grid
 // and tile) and the launches over a job table (E, jobs: device arrays).
 void member_jobs_voxel(const Dev& d, MemberJobs& mj);

@@ -975,6 +975,27 @@ void launch_cell2node(const Dev& d, double tdot, int ideriv, cudaStream_t st) {
     k_cell2node<<<d.grid, kBlock, 0, st>>>(d, tdot, ideriv);
 }
 
+// ---------------------------------------------------------------- k_interleave
+// One thread per output value: writes are contiguous, and the reads of a warp take whole 32-byte
+// sectors of each plane.  Bound by the copy to the host that follows (PCIe), not by HBM.
+struct InterleaveMap {
+    unsigned char c[kMaxInterleave];
+};
+__global__ void __launch_bounds__(kBlock) k_interleave(const double* __restrict__ in, InterleaveMap map, int nout, long long N,
+                                                        long long total, double* __restrict__ out) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+        const long long v = i / nout;
+        out[i] = in[(long long)map.c[(int)(i - v * nout)] * N + v];
+    }
+}
+void launch_interleave(const Dev& d, const double* in, const int* map, int nout, long long v0, long long nv, double* out,
+                       cudaStream_t st) {
+    InterleaveMap m{};
+    for (int c = 0; c < nout; c++) m.c[c] = (unsigned char)map[c];
+    const long long total = nv * nout, blocks = (total + kBlock - 1) / kBlock;
+    k_interleave<<<(int)(blocks < 148LL * 64 ? blocks : 148LL * 64), kBlock, 0, st>>>(in + v0, m, nout, d.N, total, out);
+}
+
 // ---------------------------------------------------------------- k_goperr0
 __device__ __forceinline__ void spatial_freq(int kx, int ky, int kz, int n1, int n2, int n3, double* xi) {
     const double twopi = 2.0 * EVP_PI;

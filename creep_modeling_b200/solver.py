@@ -88,12 +88,17 @@ class Solve:
         return r, d
 
     def field(self, name: str) -> np.ndarray:
-        cap = self.nvox * 128 + 3 * (self.shape[0] + 1) * (self.shape[1] + 1) * (self.shape[2] + 1)
-        buf = np.zeros(cap)
-        n = ctypes.c_longlong(0)
-        _lib.check(_lib.load().evp_get_field(self._h, name.encode(), buf.ctypes.data_as(ctypes.POINTER(ctypes.c_double)), cap,
-                                             ctypes.byref(n)))
-        return buf[: n.value].copy()
+        lib, n, one = _lib.load(), ctypes.c_longlong(-1), np.empty(1)
+        dp = ctypes.POINTER(ctypes.c_double)
+        # a buffer of one value: the call says how many the field has (or that it has none of that name)
+        rc = lib.evp_get_field(self._h, name.encode(), one.ctypes.data_as(dp), 1, ctypes.byref(n))
+        if rc == 0:
+            return one[: n.value]
+        if n.value < 0:
+            _lib.check(rc)
+        buf = np.empty(n.value)
+        _lib.check(lib.evp_get_field(self._h, name.encode(), buf.ctypes.data_as(dp), buf.size, ctypes.byref(n)))
+        return buf
 
     def kernel_times(self) -> dict:
         """{kernel: (launches, total ms)} recorded under ``profile=True``."""

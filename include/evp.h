@@ -73,7 +73,8 @@ int evp_advance(evp_solve* s, int nmacro, int* done);
  * components innermost, 3x3 tensors row-major).  Names: sg, sgt, velgrad,
  * velgradold, defgrad, defgradinv, defgrade, defgradp, edotp, ept,
  * disgradsym, dvelgradref, gamdot, crss, trialtau, sch, c066mod, sg66, detF,
- * wgtc, gacumgr, epvm, xnode.  *written = number of doubles copied. */
+ * wgtc, gacumgr, epvm, xnode.  *written = number of doubles copied; a buffer that
+ * is too small is refused (-7) and *written says how many the field has. */
 int evp_get_field(evp_solve* s, const char* name, double* host_out, long long capacity, long long* written);
 
 /* Last results.csv row (51 values, IO_functions.f90:1264-1271 order) and
