@@ -79,7 +79,7 @@ struct Dev {
     long long N;
     int n1, n2, n3, n1h, n3node;
     int nsys;  // max nsyst over phases (array stride of the per-system fields)
-    int grid;  // blocks of the voxel kernels
+    int grid, block;  // blocks of the voxel kernels and their threads
     double wgt;
     // voxel state
     double *sg, *sgt, *edotp, *ept, *disgradsym;         // s6

@@ -18,6 +18,7 @@
 // the same passes with a different z operator.
 #include "evp_dev.cuh"
 #include "evp_math.cuh"
+#include "evp_vox.cuh"
 
 #include <algorithm>
 #include <cstdlib>
@@ -696,46 +697,15 @@ __device__ __forceinline__ void body_fft_x_inv(const Dev& d, const FftPlan1D& pl
     }
     (void)invN;
     if (mode != 0) return;
-    // block partials -> the last block forms du = (dvelgradavg - <dL_ref F^{-1}>) inv(<F^{-1}>)
-    __shared__ double sh[9][32];
-    __shared__ bool last;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-#pragma unroll
-    for (int f = 0; f < 9; f++) {
-        double x = acc[f];
-        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-        if (lane == 0) sh[f][warp] = x;
-    }
-    __syncthreads();
-    if (warp == 0) {
-        for (int f = 0; f < 9; f++) {
-            double x = lane < nw ? sh[f][lane] : 0.0;
-            for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-            if (lane == 0) d.partials[(size_t)f * vb.nx + vb.x] = x;
-        }
-    }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) last = (atomicAdd(d.counters + CNT_XINV, 1u) == (unsigned)vb.nx - 1u);
-    __syncthreads();
+    // the last block forms du = (dvelgradavg - <dL_ref F^{-1}>) inv(<F^{-1}>)
     __shared__ double fsum[9];
-    if (last) {  // fold the block partials: one warp per field, fixed order
-        __threadfence();
-        for (int f = warp; f < 9; f += nw) {
-            const double x = fold_sum(d.partials, vb.nx, f, lane);
-            if (lane == 0) fsum[f] = x;
-        }
-        __syncthreads();
-    }
-    if (last && threadIdx.x == 0) {
-        double fl[9], dd[9], du[9];
-        for (int f = 0; f < 9; f++) {
-            fl[f] = fsum[f];
-            dd[f] = xp.dvelgradavg[f] - fl[f];
-        }
+    if (!reduce_store<9, 0>(acc, nullptr, d.partials, fsum, d.counters + CNT_XINV, vb)) return;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double dd[9], du[9];
+        for (int f = 0; f < 9; f++) dd[f] = xp.dvelgradavg[f] - fsum[f];
         mm3(dd, xp.dinv, du);
         for (int f = 0; f < 9; f++) d.red[OFF_DU + f] = du[f];
-        d.counters[CNT_XINV] = 0;
     }
 }
 template <int RS, class CT>

@@ -116,7 +116,7 @@ void launch_init(const Dev& d, const double* euler, const int* grain, const doub
     for (int c = 0; c < 6; c++) ip.u6t[c] = u6t[c];
     ip.keepF = keepF;
     ip.detFavg = detFavg;
-    k_init<<<d.grid, kBlock, 0, st>>>(d, euler, grain, hp, ip);
+    k_init<<<d.grid, d.block, 0, st>>>(d, euler, grain, hp, ip);
 }
 
 // ---------------------------------------------------------------- k_dispini
@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(kBlock) k_dispini(Dev d, const double* __restr
     reduce_store<30, 0>(sums, nullptr, d.partials, d.red + OFF_DISP, d.counters + CNT_DISP, hw_vb());
 }
 void launch_dispini(const Dev& d, const double* grad, double delt, cudaStream_t st) {
-    k_dispini<<<d.grid, kBlock, 0, st>>>(d, grad, delt);
+    k_dispini<<<d.grid, d.block, 0, st>>>(d, grad, delt);
 }
 
 // ---------------------------------------------------------------- k_sgavg
@@ -168,7 +168,7 @@ __device__ __forceinline__ void body_sgavg(const Dev& d, const VB& vb) {
     reduce_store<6, 0>(s, nullptr, d.partials, d.red + OFF_SGAVG, d.counters + CNT_SGAVG, vb);
 }
 __global__ void __launch_bounds__(kBlock) k_sgavg(Dev d) { body_sgavg(d, hw_vb()); }
-void launch_sgavg(const Dev& d, cudaStream_t st) { k_sgavg<<<d.grid, kBlock, 0, st>>>(d); }
+void launch_sgavg(const Dev& d, cudaStream_t st) { k_sgavg<<<d.grid, d.block, 0, st>>>(d); }
 
 // ---------------------------------------------------------------- b-basis congruence
 // For a 3x3 matrix M, T(M)_ag = <B^a, B^g M^T> (Frobenius product; B^0..B^5 the orthonormal
@@ -320,8 +320,8 @@ __global__ void __launch_bounds__(kBlock, 2) k_prologue_modal(Dev d, const doubl
     }
 }
 void launch_prologue(const Dev& d, const double* c0, const double* goperr0, int do_schmid, int modal, cudaStream_t st) {
-    k_prologue<<<d.grid, kBlock, 0, st>>>(d, c0, goperr0, do_schmid, modal);
-    if (modal) k_prologue_modal<<<d.grid, kBlock, 0, st>>>(d, goperr0);
+    k_prologue<<<d.grid, d.block, 0, st>>>(d, c0, goperr0, do_schmid, modal);
+    if (modal) k_prologue_modal<<<d.grid, d.block, 0, st>>>(d, goperr0);
 }
 
 // ---------------------------------------------------------------- k_gas_compl
@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(kBlock) k_gas_compl(Dev d, double tdot, double
     }
 }
 void launch_gas_compl(const Dev& d, double tdot, double complgas, int modal, cudaStream_t st) {
-    k_gas_compl<<<d.grid, kBlock, 0, st>>>(d, tdot, complgas, modal);
+    k_gas_compl<<<d.grid, d.block, 0, st>>>(d, tdot, complgas, modal);
 }
 
 // ---------------------------------------------------------------- k_corr
@@ -401,7 +401,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_corr(Dev d, CorrParams p) {
 // 31-field block reduction over more loads
 void launch_corr(const Dev& d, const CorrParams& p, cudaStream_t st) {
     const int grid = d.grid < 148 * 2 ? d.grid : 148 * 2;
-    k_corr<<<grid, kBlock, 0, st>>>(d, p);
+    k_corr<<<grid, d.block, 0, st>>>(d, p);
 }
 
 // ---------------------------------------------------------------- batched launches of the iteration's voxel passes
@@ -430,7 +430,8 @@ void member_jobs_voxel(const Dev& d, MemberJobs& mj) {
         mj.smem[0][k] = sm;
         mj.variant[0][k] = variant;
     };
-    one_d(BK_CORR, d.grid < 148 * 2 ? d.grid : 148 * 2, kBlock, 0, d.cgas ? 0 : 1);
+    // members of one block size share a launch: variant = (no gas phase) + 2 * (block size / 32)
+    one_d(BK_CORR, d.grid < 148 * 2 ? d.grid : 148 * 2, d.block, 0, (d.cgas ? 0 : 1) + 2 * (d.block / 32));
     const NewtonShape n = newton_shape(d);
     one_d(BK_NEWTON, n.grid, n.threads, n.smem, n.variant);
 }
@@ -438,7 +439,7 @@ void member_jobs_voxel(const Dev& d, MemberJobs& mj) {
 void launch_batched_voxel(const BatchLaunch& L, const BatchParams& P, cudaStream_t st) {
     switch (L.kind) {
         case BK_CORR:
-            if (L.variant == 0) kb_corr<true><<<L.blocks, L.threads, 0, st>>>(P);
+            if ((L.variant & 1) == 0) kb_corr<true><<<L.blocks, L.threads, 0, st>>>(P);
             else kb_corr<false><<<L.blocks, L.threads, 0, st>>>(P);
             break;
         case BK_NEWTON:
@@ -528,8 +529,8 @@ __global__ void __launch_bounds__(kBlock) k_upd1(Dev d, Upd1Params p) {
     reduce_store<39, 1>(s, mx, d.partials, d.red + OFF_UPD1, d.counters + CNT_UPD1, hw_vb());
 }
 void launch_upd1(const Dev& d, const Upd1Params& p, cudaStream_t st) {
-    if (d.nsys <= 12) k_upd1<12><<<d.grid, kBlock, 0, st>>>(d, p);
-    else k_upd1<24><<<d.grid, kBlock, 0, st>>>(d, p);
+    if (d.nsys <= 12) k_upd1<12><<<d.grid, d.block, 0, st>>>(d, p);
+    else k_upd1<24><<<d.grid, d.block, 0, st>>>(d, p);
 }
 
 // ---------------------------------------------------------------- k_upd2
@@ -617,51 +618,20 @@ __global__ void __launch_bounds__(kBlock) k_upd2(Dev d, Upd2Params p) {
 #pragma unroll
         for (int c = 0; c < 9; c++) s[c] += vg[c] * w;
     }
-    // reduce; the last block forms du2 = (<L>_prev - <L>) inv(<F^{-1}>_c)
-    __shared__ double sh[9][32];
-    __shared__ bool last;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-#pragma unroll
-    for (int f = 0; f < 9; f++) {
-        double x = s[f];
-        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-        if (lane == 0) sh[f][warp] = x;
-    }
-    __syncthreads();
-    if (warp == 0) {
-        for (int f = 0; f < 9; f++) {
-            double x = lane < nw ? sh[f][lane] : 0.0;
-            for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-            if (lane == 0) d.partials[(size_t)f * gridDim.x + blockIdx.x] = x;
-        }
-    }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) last = (atomicAdd(d.counters + CNT_UPD2, 1u) == gridDim.x - 1);
-    __syncthreads();
+    // the last block forms du2 = (<L>_prev - <L>) inv(<F^{-1}>_c)
     __shared__ double fsum[9];
-    if (last) {
-        __threadfence();
-        for (int f = warp; f < 9; f += nw) {
-            const double x = fold_sum(d.partials, gridDim.x, f, lane);
-            if (lane == 0) fsum[f] = x;
-        }
-        __syncthreads();
-    }
-    if (last && threadIdx.x == 0) {
-        double va[9], fc[9], di[9], dd[9], du[9];
-        for (int f = 0; f < 9; f++) {
-            va[f] = fsum[f];
-            fc[f] = __ldcg(&d.red[OFF_UPD1 + 9 + f]) / dav;
-        }
+    if (!reduce_store<9, 0>(s, nullptr, d.partials, fsum, d.counters + CNT_UPD2, hw_vb())) return;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double fc[9], di[9], dd[9], du[9];
+        for (int f = 0; f < 9; f++) fc[f] = __ldcg(&d.red[OFF_UPD1 + 9 + f]) / dav;
         if (inv3u(fc, di) != 0) set_err(d.err, 1);
-        for (int f = 0; f < 9; f++) dd[f] = p.velgradavg[f] - va[f];
+        for (int f = 0; f < 9; f++) dd[f] = p.velgradavg[f] - fsum[f];
         mm3(dd, di, du);
         for (int f = 0; f < 9; f++) d.red[OFF_DU2 + f] = du[f];
-        d.counters[CNT_UPD2] = 0;
     }
 }
-void launch_upd2(const Dev& d, const Upd2Params& p, cudaStream_t st) { k_upd2<<<d.grid, kBlock, 0, st>>>(d, p); }
+void launch_upd2(const Dev& d, const Upd2Params& p, cudaStream_t st) { k_upd2<<<d.grid, d.block, 0, st>>>(d, p); }
 
 // ---------------------------------------------------------------- k_upd3
 template <int NS>
@@ -738,8 +708,8 @@ __global__ void __launch_bounds__(kBlock, 2) k_upd3(Dev d, Upd3Params p) {
     reduce_store<30, 0>(s, nullptr, d.partials, d.red + OFF_UPD3, d.counters + CNT_UPD3, hw_vb());
 }
 void launch_upd3(const Dev& d, const Upd3Params& p, cudaStream_t st) {
-    if (d.nsys <= 12) k_upd3<12><<<d.grid, kBlock, 0, st>>>(d, p);
-    else k_upd3<24><<<d.grid, kBlock, 0, st>>>(d, p);
+    if (d.nsys <= 12) k_upd3<12><<<d.grid, d.block, 0, st>>>(d, p);
+    else k_upd3<24><<<d.grid, d.block, 0, st>>>(d, p);
 }
 
 // ---------------------------------------------------------------- k_diag
@@ -800,23 +770,25 @@ __global__ void __launch_bounds__(kBlock, 2) k_diag(Dev d, double Lfloor) {
         }
     }
     // (min, last index) pairs reduced first, by a fixed-order warp/block tree
-    __shared__ MinIdx shm[2][32];
+    __shared__ MinIdx shm[2][8];
     __shared__ bool lastblk;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int o = 16; o > 0; o >>= 1) {
-        MinIdx a = {__shfl_down_sync(0xffffffffu, ms.v, o), __shfl_down_sync(0xffffffffu, ms.i, o)};
-        MinIdx b = {__shfl_down_sync(0xffffffffu, mg.v, o), __shfl_down_sync(0xffffffffu, mg.i, o)};
-        ms = min_last(ms, a);
-        mg = min_last(mg, b);
-    }
-    if (lane == 0) { shm[0][warp] = ms; shm[1][warp] = mg; }
-    __syncthreads();
+    auto block_min = [&](MinIdx& x, MinIdx& y) {  // the result is in thread 0
+        for (int o = 16; o > 0; o >>= 1) {
+            x = min_last(x, MinIdx{__shfl_down_sync(0xffffffffu, x.v, o), __shfl_down_sync(0xffffffffu, x.i, o)});
+            y = min_last(y, MinIdx{__shfl_down_sync(0xffffffffu, y.v, o), __shfl_down_sync(0xffffffffu, y.i, o)});
+        }
+        __syncthreads();
+        if (lane == 0) { shm[0][warp] = x; shm[1][warp] = y; }
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int q = 0; q < nw; q++) { x = min_last(x, shm[0][q]); y = min_last(y, shm[1][q]); }
+    };
+    block_min(ms, mg);
     MinIdx* pm = reinterpret_cast<MinIdx*>(d.partials + (size_t)gridDim.x * 19);
     if (threadIdx.x == 0) {
-        MinIdx a = shm[0][0], b = shm[1][0];
-        for (int q = 1; q < nw; q++) { a = min_last(a, shm[0][q]); b = min_last(b, shm[1][q]); }
-        pm[2 * blockIdx.x] = a;
-        pm[2 * blockIdx.x + 1] = b;
+        pm[2 * blockIdx.x] = ms;
+        pm[2 * blockIdx.x + 1] = mg;
     }
     __syncthreads();
     reduce_store<6, 13>(s, m, d.partials, d.red + OFF_DIAG, d.counters + CNT_DIAG, hw_vb());
@@ -825,37 +797,26 @@ __global__ void __launch_bounds__(kBlock, 2) k_diag(Dev d, double Lfloor) {
     __syncthreads();
     if (threadIdx.x == 0) lastblk = (atomicAdd(d.counters + CNT_DIAG2, 1u) == gridDim.x - 1);
     __syncthreads();
-    if (lastblk && threadIdx.x == 0) {
-        __threadfence();
-        MinIdx a = {EVP_HUGE, -1}, b = {EVP_HUGE, -1};
-        unsigned q = 0;
-        for (; q + 8 <= gridDim.x; q += 8) {  // eight blocks' pairs loaded at a time, folded in block order
-            MinIdx x[8], y[8];
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                x[i] = MinIdx{__ldcg(&pm[2 * (q + i)].v), __ldcg(&pm[2 * (q + i)].i)};
-                y[i] = MinIdx{__ldcg(&pm[2 * (q + i) + 1].v), __ldcg(&pm[2 * (q + i) + 1].i)};
-            }
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                a = min_last(a, x[i]);
-                b = min_last(b, y[i]);
-            }
-        }
-        for (; q < gridDim.x; q++) {
-            MinIdx x = {__ldcg(&pm[2 * q].v), __ldcg(&pm[2 * q].i)};
-            MinIdx y = {__ldcg(&pm[2 * q + 1].v), __ldcg(&pm[2 * q + 1].i)};
-            a = min_last(a, x);
-            b = min_last(b, y);
-        }
-        d.red[OFF_DIAG + 19] = a.v;
-        d.red[OFF_DIAG + 20] = (double)a.i;
-        d.red[OFF_DIAG + 21] = b.v;
-        d.red[OFF_DIAG + 22] = (double)b.i;
+    if (!lastblk) return;
+    // the block pairs: every thread folds some (any order gives the same pair: the smallest value, and
+    // of its voxels the last), then the block
+    __threadfence();
+    ms = MinIdx{EVP_HUGE, -1};
+    mg = MinIdx{EVP_HUGE, -1};
+    for (unsigned q = threadIdx.x; q < gridDim.x; q += blockDim.x) {
+        ms = min_last(ms, MinIdx{__ldcg(&pm[2 * q].v), __ldcg(&pm[2 * q].i)});
+        mg = min_last(mg, MinIdx{__ldcg(&pm[2 * q + 1].v), __ldcg(&pm[2 * q + 1].i)});
+    }
+    block_min(ms, mg);
+    if (threadIdx.x == 0) {
+        d.red[OFF_DIAG + 19] = ms.v;
+        d.red[OFF_DIAG + 20] = (double)ms.i;
+        d.red[OFF_DIAG + 21] = mg.v;
+        d.red[OFF_DIAG + 22] = (double)mg.i;
         d.counters[CNT_DIAG2] = 0;
     }
 }
-void launch_diag(const Dev& d, double Lfloor, cudaStream_t st) { k_diag<<<d.grid, kBlock, 0, st>>>(d, Lfloor); }
+void launch_diag(const Dev& d, double Lfloor, cudaStream_t st) { k_diag<<<d.grid, d.block, 0, st>>>(d, Lfloor); }
 
 // ---------------------------------------------------------------- k_c0
 template <int NS>
@@ -932,7 +893,7 @@ __global__ void __launch_bounds__(kBlock) k_kinematic(Dev d, double tdot_step) {
     }
     reduce_store<0, 4>(nullptr, m, d.partials, d.red + OFF_KIN, d.counters + CNT_KIN, hw_vb());
 }
-void launch_kinematic(const Dev& d, double tdot_step, cudaStream_t st) { k_kinematic<<<d.grid, kBlock, 0, st>>>(d, tdot_step); }
+void launch_kinematic(const Dev& d, double tdot_step, cudaStream_t st) { k_kinematic<<<d.grid, d.block, 0, st>>>(d, tdot_step); }
 
 // ---------------------------------------------------------------- k_cell2node
 __global__ void __launch_bounds__(kBlock) k_cell2node(Dev d, double tdot, int ideriv) {
@@ -972,7 +933,7 @@ __global__ void __launch_bounds__(kBlock) k_cell2node(Dev d, double tdot, int id
     }
 }
 void launch_cell2node(const Dev& d, double tdot, int ideriv, cudaStream_t st) {
-    k_cell2node<<<d.grid, kBlock, 0, st>>>(d, tdot, ideriv);
+    k_cell2node<<<d.grid, d.block, 0, st>>>(d, tdot, ideriv);
 }
 
 // ---------------------------------------------------------------- k_interleave
@@ -1147,7 +1108,7 @@ __global__ void __launch_bounds__(kBlock) k_goperr0(Dev d, const double* __restr
     reduce_store<81, 0>(s, nullptr, d.partials, d.red + OFF_G0, d.counters + CNT_G0, hw_vb());
 }
 void launch_goperr0(const Dev& d, const double* c0, const double* s0, int igamma, cudaStream_t st) {
-    k_goperr0<<<d.grid, kBlock, 0, st>>>(d, c0, s0, igamma);
+    k_goperr0<<<d.grid, d.block, 0, st>>>(d, c0, s0, igamma);
 }
 
 // form_G for IGAMMA 1 and 2 on the half spectrum, once per increment (c0 changes per increment)
@@ -1166,7 +1127,7 @@ __global__ void __launch_bounds__(kBlock) k_goper_tab(Dev d, const double* __res
     }
 }
 void launch_goper_tab(const Dev& d, const double* c0, const double* s0, int igamma, cudaStream_t st) {
-    k_goper_tab<<<d.grid, kBlock, 0, st>>>(d, c0, s0, igamma);
+    k_goper_tab<<<d.grid, d.block, 0, st>>>(d, c0, s0, igamma);
 }
 
 }  // namespace evp

@@ -381,36 +381,15 @@ __device__ __forceinline__ void gas_voxel(const Dev& d, const NewtonParams& p, l
     for (int q = 0; q < d.nsys; q++) d.gamdot[q * N + v] = 0.0;
 }
 
-// Sums of eight values over the warp by halving exchanges (nine shuffles of a double): lanes
-// 4 q .. 4 q + 3 end with the sum of value sum8_field(lane).
-__device__ __forceinline__ int sum8_field(int lane) { return ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1); }
-__device__ __forceinline__ double warp_sum8(double (&x)[8], int lane) {
-#pragma unroll
-    for (int h = 4; h >= 1; h /= 2) {
-        const bool up = lane & (4 * h);
-#pragma unroll
-        for (int f = 0; f < h; f++) {
-            const double send = up ? x[f] : x[f + h], keep = up ? x[f + h] : x[f];
-            x[f] = keep + __shfl_xor_sync(0xffffffffu, send, 4 * h);
-        }
-    }
-    double y = x[0];
-    y += __shfl_xor_sync(0xffffffffu, y, 2);
-    y += __shfl_xor_sync(0xffffffffu, y, 1);
-    return y;
-}
-
 // Every warp of the block has put its 14 sums into sh -> one partial per block -> the last block
-// folds them in block order; a block of few warps folds its fields together so that their loads
-// overlap.
+// folds them in block order (reduce_store's second half, with running sums per warp before it).
 constexpr int kNewtonSums = 14;
 __device__ __forceinline__ void reduce_newton(const double (*sh)[kNewtonSums], double* partials, double* out, unsigned int* counter,
                                               const VB& vb) {
-    constexpr int NF = kNewtonSums;
     __shared__ bool last;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
     __syncthreads();
-    if (threadIdx.x < NF) {
+    if (threadIdx.x < kNewtonSums) {
         double x = sh[0][threadIdx.x];
         for (int w = 1; w < nw; w++) x += sh[w][threadIdx.x];
         partials[(size_t)threadIdx.x * vb.nx + vb.x] = x;
@@ -421,26 +400,7 @@ __device__ __forceinline__ void reduce_newton(const double (*sh)[kNewtonSums], d
     __syncthreads();
     if (!last) return;
     __threadfence();
-    if (nw >= 4) {
-        for (int f = warp; f < NF; f += nw) {
-            const double x = fold_sum(partials, vb.nx, f, lane);
-            if (lane == 0) out[f] = x;
-        }
-    } else if (warp == 0) {
-        double s[NF];
-#pragma unroll
-        for (int f = 0; f < NF; f++) s[f] = 0.0;
-        for (int b = lane; b < vb.nx; b += 32)
-#pragma unroll
-            for (int f = 0; f < NF; f++) s[f] += __ldcg(partials + (size_t)f * vb.nx + b);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-            for (int f = 0; f < NF; f++) s[f] += __shfl_down_sync(0xffffffffu, s[f], o);
-        if (lane == 0)
-#pragma unroll
-            for (int f = 0; f < NF; f++) out[f] = s[f];
-    }
+    for (int f = warp; f < kNewtonSums; f += 4 * nw) fold_four<false>(partials, vb.nx, f, nw, kNewtonSums, out, lane);
     if (threadIdx.x == 0) *counter = 0;
 }
 
@@ -492,7 +452,7 @@ __device__ __forceinline__ void body_newtonv(const Dev& d, const NewtonParams& p
     const double tolt = fmax(p.error, p.erroral), idt = 1.0 / p.tdot;
     const bool stats = d.nstats != nullptr;
     unsigned c_pass = 0, c_eval = 0, c_nr = 0, c_tau = 0, c_vox = 0, c_npass = 0;
-    double mine = 0.0, mineg = 0.0;  // running sum sum8_field(lane) of this warp: dsg and ddg norms, stress (solid; gas)
+    double mine = 0.0, mineg = 0.0;  // running sum lane / 4 of this warp: dsg and ddg norms, stress (solid; gas)
     const long long stride = (long long)vb.nx * blockDim.x;
     for (long long v0 = (long long)vb.x * blockDim.x + (threadIdx.x & ~31); v0 < N; v0 += stride) {  // warp-uniform
         const long long v = v0 + lane;
@@ -799,8 +759,8 @@ __device__ __forceinline__ void body_newtonv(const Dev& d, const NewtonParams& p
             }
         }
         __syncwarp();
-        mine += warp_sum8(sums, lane);
-        if (d.cgas) mineg += warp_sum8(gsum, lane);
+        mine += warp_reduce_many<8, false>(sums, lane);
+        if (d.cgas) mineg += warp_reduce_many<8, false>(gsum, lane);
     }
     if (stats) {
         unsigned c[6] = {c_pass, c_eval, c_nr, c_tau, c_vox, c_npass};
@@ -813,7 +773,7 @@ __device__ __forceinline__ void body_newtonv(const Dev& d, const NewtonParams& p
     // dsg and ddg norms, the solid's stress sum and the whole cell's
     __shared__ double sh[8][kNewtonSums];
     if ((lane & 3) == 0) {
-        const int f = sum8_field(lane);
+        const int f = lane >> 2;
         sh[threadIdx.x >> 5][f] = mine;
         if (f >= 2) sh[threadIdx.x >> 5][f + 6] = mine + mineg;
     }

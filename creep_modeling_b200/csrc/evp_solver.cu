@@ -380,8 +380,11 @@ public:
         int ns = 1;
         for (auto& ph : dk.phase) ns = std::max(ns, ph.nsyst);
         d.nsys = ns;
-        long long g = (N + 255) / 256;
-        d.grid = (int)std::min<long long>(g, 148LL * 8);
+        // blocks of 256, smaller ones where those would leave SMs without a block (16^3: 64 blocks
+        // of 64 instead of 16 of 256), not below two warps, whose fold of the block sums takes longer
+        d.block = 256;
+        while (d.block > 64 && (N + d.block - 1) / d.block < 148) d.block /= 2;
+        d.grid = (int)std::min<long long>((N + d.block - 1) / d.block, 148LL * 8);
         d.sg = dalloc<double>(6 * N); d.sgt = dalloc<double>(6 * N); d.edotp = dalloc<double>(6 * N);
         d.ept = dalloc<double>(6 * N); d.disgradsym = dalloc<double>(6 * N);
         d.velgrad = dalloc<double>(9 * N); d.velgradold = dalloc<double>(9 * N); d.dvr = dalloc<double>(9 * N);

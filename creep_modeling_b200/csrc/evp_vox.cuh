@@ -12,68 +12,115 @@ constexpr int kC0Block = 64;
 
 // ---------------------------------------------------------------- reductions
 // NS sums then NM maxima per thread -> one partial per block (stored field-major,
-// partials[f * nblocks + block], in the body's block coordinates) -> the last block to finish folds them: one
-// warp per field, lane l adding blocks l, l + 32, ... in order, then a fixed
-// shuffle tree, so the result does not depend on timing (fold_sum, in evp_dev.cuh, for the
-// sums; fold_max for the maxima).
-__device__ __forceinline__ double fold_max(const double* partials, int nblk, int f, int lane) {
-    const double* q = partials + (size_t)f * nblk;
-    double s = -EVP_HUGE;
-    int b = lane;
-    for (; b + 7 * 32 < nblk; b += 8 * 32) {
-        double x[8];
+// partials[f * nblocks + block], in the body's block coordinates) -> the last block to finish
+// folds them: lane l of a field's warp adds blocks l, l + 32, ... in order, then a fixed shuffle
+// tree, so the result does not depend on timing.
+//
+// On small grids this is most of a pass, and it is all latency, so nothing goes one field at a
+// time: a warp reduces 32 fields by halving exchanges (31 shuffles instead of 160; lane f ends
+// with field f), the block's warps are added by a thread per field, and the last block's warps
+// fold four fields each at once.  Event-timed launches, with blocks of 64 at 16^3 instead of 256:
+// k_corr 15.9 -> 13.8 us, k_fft_x_inv 15.8 -> 13.8, k_c0 (72 sums) 74 -> 47 (an empty launch reads
+// 5 us); at 64^3 k_corr 31.6 -> 25.4, k_fft_x_inv 39 -> 36, k_c0 500 -> 434, and k_diag 240 -> 132,
+// whose block pairs one thread used to fold.
+template <bool MAX>
+__device__ __forceinline__ double red_op(double a, double b) { return MAX ? fmax(a, b) : a + b; }
+
+// W (a power of two, at most 32) values over the warp: lane l ends with value l >> (5 - log2 W)
+template <int W, bool MAX>
+__device__ __forceinline__ double warp_reduce_many(double (&x)[W], int lane) {
+    int dist = 16;
 #pragma unroll
-        for (int i = 0; i < 8; i++) x[i] = __ldcg(q + b + 32 * i);
+    for (int h = W / 2; h >= 1; h /= 2, dist /= 2) {
+        const bool up = lane & dist;
 #pragma unroll
-        for (int i = 0; i < 8; i++) s = fmax(s, x[i]);
+        for (int f = 0; f < h; f++) {
+            const double send = up ? x[f] : x[f + h], keep = up ? x[f + h] : x[f];
+            x[f] = red_op<MAX>(keep, __shfl_xor_sync(0xffffffffu, send, dist));
+        }
     }
-    for (; b < nblk; b += 32) s = fmax(s, __ldcg(q + b));
+    double y = x[0];
+    for (; dist >= 1; dist /= 2) y = red_op<MAX>(y, __shfl_xor_sync(0xffffffffu, y, dist));
+    return y;
+}
+__host__ __device__ constexpr int pow2_at_least(int n) { return n <= 1 ? 1 : 2 * pow2_at_least((n + 1) / 2); }
+__host__ __device__ constexpr int log2_of(int n) { return n <= 1 ? 0 : 1 + log2_of(n / 2); }
+// fields [F0, F0 + NF) of the thread's values into sh[f] (one row per warp)
+template <int NF, bool MAX, int F0 = 0>
+__device__ __forceinline__ void warp_fields(const double* vals, double* sh, int lane) {
+    if constexpr (F0 < NF) {
+        constexpr int n = NF - F0 < 32 ? NF - F0 : 32, W = pow2_at_least(n);
+        double x[W];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s = fmax(s, __shfl_down_sync(0xffffffffu, s, o));
-    return s;  // in lane 0
+        for (int f = 0; f < W; f++) x[f] = f < n ? vals[F0 + f] : (MAX ? -EVP_HUGE : 0.0);
+        const double y = warp_reduce_many<W, MAX>(x, lane);
+        constexpr int sft = 5 - log2_of(W);
+        if ((lane & ((1 << sft) - 1)) == 0 && (lane >> sft) < n) sh[F0 + (lane >> sft)] = y;
+        warp_fields<NF, MAX, F0 + 32>(vals, sh, lane);
+    }
+}
+// fold of fields f0, f0 + step, f0 + 2 step, f0 + 3 step (below nf) over the block partials by one warp
+template <bool MAX>
+__device__ __forceinline__ void fold_four(const double* partials, int nblk, int f0, int step, int nf, double* out, int lane) {
+    double s[4];
+    const double* q[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        s[i] = MAX ? -EVP_HUGE : 0.0;
+        q[i] = partials + (size_t)(f0 + i * step < nf ? f0 + i * step : f0) * nblk;
+    }
+    int b = lane;
+    for (; b + 3 * 32 < nblk; b += 4 * 32) {
+        double x[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) x[i][j] = __ldcg(q[i] + b + 32 * j);
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) s[i] = red_op<MAX>(s[i], x[i][j]);
+    }
+    for (; b < nblk; b += 32)
+#pragma unroll
+        for (int i = 0; i < 4; i++) s[i] = red_op<MAX>(s[i], __ldcg(q[i] + b));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int i = 0; i < 4; i++) s[i] = red_op<MAX>(s[i], __shfl_down_sync(0xffffffffu, s[i], o));
+    if (lane == 0)
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            if (f0 + i * step < nf) out[f0 + i * step] = s[i];
 }
 
+// Returns true in every thread of the block that folded (out is then written, visible to the
+// block after a __syncthreads); blocks of at most 8 warps, whole warps.
 template <int NS, int NM>
-__device__ void reduce_store(const double* sums, const double* maxs, double* partials, double* out, unsigned int* counter,
+__device__ bool reduce_store(const double* sums, const double* maxs, double* partials, double* out, unsigned int* counter,
                              const VB& vb) {
     constexpr int NF = NS + NM;
-    __shared__ double sh[NF][32];
+    __shared__ double sh[8][NF];
     __shared__ bool last;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-#pragma unroll
-    for (int f = 0; f < NF; f++) {
-        double x = (f < NS) ? sums[f] : maxs[f - NS];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            double y = __shfl_down_sync(0xffffffffu, x, o);
-            x = (f < NS) ? x + y : fmax(x, y);
-        }
-        if (lane == 0) sh[f][warp] = x;
-    }
+    warp_fields<NS, false>(sums, sh[warp], lane);
+    warp_fields<NM, true>(maxs, sh[warp] + NS, lane);
     __syncthreads();
-    if (warp == 0) {
-        for (int f = 0; f < NF; f++) {
-            double x = (lane < nw) ? sh[f][lane] : ((f < NS) ? 0.0 : -EVP_HUGE);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                double y = __shfl_down_sync(0xffffffffu, x, o);
-                x = (f < NS) ? x + y : fmax(x, y);
-            }
-            if (lane == 0) partials[(size_t)f * vb.nx + vb.x] = x;
-        }
+    for (int f = threadIdx.x; f < NF; f += blockDim.x) {
+        double x = sh[0][f];
+        for (int w = 1; w < nw; w++) x = f < NS ? x + sh[w][f] : fmax(x, sh[w][f]);
+        partials[(size_t)f * vb.nx + vb.x] = x;
     }
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) last = (atomicAdd(counter, 1u) == (unsigned)vb.nx - 1u);
     __syncthreads();
-    if (last) {
-        __threadfence();
-        for (int f = warp; f < NF; f += nw) {
-            const double x = (f < NS) ? fold_sum(partials, vb.nx, f, lane) : fold_max(partials, vb.nx, f, lane);
-            if (lane == 0) out[f] = x;
-        }
-        if (threadIdx.x == 0) *counter = 0;
-    }
+    if (!last) return false;
+    __threadfence();
+    for (int f = warp; f < NS; f += 4 * nw) fold_four<false>(partials, vb.nx, f, nw, NS, out, lane);
+    for (int f = NS + warp; f < NF; f += 4 * nw) fold_four<true>(partials, vb.nx, f, nw, NF, out, lane);
+    if (threadIdx.x == 0) *counter = 0;
+    return true;
 }
 
 __device__ __forceinline__ void set_err(int* err, int bit) { atomicOr(err, bit); }
