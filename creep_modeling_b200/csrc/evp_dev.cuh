@@ -201,7 +201,7 @@ struct Job {
 // iteration of an increment starts from is formed when the increment's iterations start).
 enum BatchKind : int { BK_XFWD, BK_YFWD, BK_ZGREEN, BK_YINV, BK_XINV, BK_CORR, BK_NEWTON, BK_N };
 struct BatchLaunch {
-    int kind, variant;  // variant: FFT passes rs | (FP32 << 1); Newton: the kernel (newton_variant)
+    int kind, variant;  // variant: FFT passes rs | (FP32 << 2); Newton: the kernel (newton_variant)
     int job0, njobs;    // slice of the plan's job table
     int blocks, threads;
     size_t smem;

@@ -28,6 +28,7 @@
 #include <sstream>
 #include <stdexcept>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 namespace evp {
@@ -63,7 +64,7 @@ template <bool INV, class CT>
 __device__ __forceinline__ CT mul_mi(CT a) { return INV ? mk<CT>(-a.y, a.x) : mk<CT>(a.y, -a.x); }
 
 template <int R, bool INV, class CT>
-__device__ __forceinline__ void dft_small(CT (&v)[R], const CT* __restrict__ tw, int n) {
+__device__ __forceinline__ void dft_small(CT (&v)[R]) {
     using T = typename CxT<CT>::T;
     if constexpr (R == 2) {
         CT a = v[0], b = v[1];
@@ -78,8 +79,8 @@ __device__ __forceinline__ void dft_small(CT (&v)[R], const CT* __restrict__ tw,
     } else if constexpr (R == 8) {
         const T c = (T)0.70710678118654752440;
         CT e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
-        dft_small<4, INV, CT>(e, tw, n);
-        dft_small<4, INV, CT>(o, tw, n);
+        dft_small<4, INV, CT>(e);
+        dft_small<4, INV, CT>(o);
         CT w1 = INV ? mk<CT>(c, c) : mk<CT>(c, -c);
         CT w3 = INV ? mk<CT>(-c, c) : mk<CT>(-c, -c);
         CT p0 = o[0], p1 = cmul(o[1], w1), p2 = mul_mi<INV, CT>(o[2]), p3 = cmul(o[3], w3);
@@ -87,67 +88,157 @@ __device__ __forceinline__ void dft_small(CT (&v)[R], const CT* __restrict__ tw,
         v[1] = cadd(e[1], p1); v[5] = csub(e[1], p1);
         v[2] = cadd(e[2], p2); v[6] = csub(e[2], p2);
         v[3] = cadd(e[3], p3); v[7] = csub(e[3], p3);
-    } else {
-        CT in[R];
-#pragma unroll
-        for (int r = 0; r < R; r++) in[r] = v[r];
-        const int step = n / R;
-#pragma unroll
-        for (int q = 0; q < R; q++) {
-            CT acc = in[0];
-#pragma unroll
-            for (int r = 1; r < R; r++) {
-                CT w = tw[((r * q) % R) * step];
-                if (INV) w.y = -w.y;
-                acc = cadd(acc, cmul(in[r], w));
-            }
-            v[q] = acc;
-        }
     }
 }
 
-// One Stockham stage over P pencils of length n stored element-major in
-// shared memory: element e of pencil p at s[e*ES + p].
-template <int R, bool INV, int MAXB, class CT>
-__device__ __forceinline__ void fft_stage(CT* s, int ES, int P, int n, int Ns, const CT* __restrict__ tw) {
+// cos and sin of 2 pi k / R, k = 1 .. (R - 1) / 2, of the odd radices
+template <int R>
+__device__ __forceinline__ double root_cos(int k) {  // k a compile-time constant after unrolling
+    if constexpr (R == 3) return -0.5;
+    if constexpr (R == 5) return k == 1 ? 0.3090169943749474241 : (-0.8090169943749474241);
+    if constexpr (R == 7) return k == 1 ? 0.62348980185873353053 : (k == 2 ? -0.22252093395631440429 : (-0.90096886790241912624));
+    if constexpr (R == 11) return k == 1 ? 0.84125353283118116886 : (k == 2 ? 0.41541501300188642553 : (k == 3 ? -0.14231483827328514044 : (k == 4 ? -0.65486073394528506406 : (-0.95949297361449738989))));
+    if constexpr (R == 13) return k == 1 ? 0.8854560256532098959 : (k == 2 ? 0.56806474673115580251 : (k == 3 ? 0.12053668025532305335 : (k == 4 ? -0.35460488704253562597 : (k == 5 ? -0.74851074817110109863 : (-0.97094181742605202716)))));
+}
+template <int R>
+__device__ __forceinline__ double root_sin(int k) {  // k a compile-time constant after unrolling
+    if constexpr (R == 3) return 0.86602540378443864676;
+    if constexpr (R == 5) return k == 1 ? 0.95105651629515357212 : (0.58778525229247312917);
+    if constexpr (R == 7) return k == 1 ? 0.78183148246802980871 : (k == 2 ? 0.97492791218182360702 : (0.43388373911755812048));
+    if constexpr (R == 11) return k == 1 ? 0.54064081745559758211 : (k == 2 ? 0.90963199535451837141 : (k == 3 ? 0.98982144188093273238 : (k == 4 ? 0.75574957435425828377 : (0.28173255684142969771))));
+    if constexpr (R == 13) return k == 1 ? 0.46472317204376854566 : (k == 2 ? 0.82298386589365639458 : (k == 3 ? 0.9927088740980539928 : (k == 4 ? 0.93501624268541482344 : (k == 5 ? 0.66312265824079520238 : (0.23931566428755776715)))));
+}
+// DFT of odd length R, its outputs handed to out(q, value) a pair at a time: with t_k = v_k + v_(R-k)
+// and u_k = v_k - v_(R-k), outputs q and R - q are A -+ i B, A = v_0 + sum_k cos(2 pi k q / R) t_k,
+// B = sum_k sin(2 pi k q / R) u_k.  Half the products of the plain sum, and no second array of R
+// values (the plain sum kept 2 R and read its roots from memory: 2 kB of spills in every all-radix kernel).
+template <int R, bool INV, class CT, class Out>
+__device__ __forceinline__ void dft_odd(CT (&v)[R], const Out& out) {
+    using T = typename CxT<CT>::T;
+    constexpr int H = (R - 1) / 2;
+    CT sum = v[0];
+#pragma unroll
+    for (int k = 1; k <= H; k++) {
+        const CT a = v[k], b = v[R - k];
+        v[k] = cadd(a, b);
+        v[R - k] = csub(a, b);
+        sum = cadd(sum, v[k]);
+    }
+    out(0, sum);
+#pragma unroll
+    for (int q = 1; q <= H; q++) {
+        CT A = v[0], B = mk<CT>(0, 0);
+#pragma unroll
+        for (int k = 1; k <= H; k++) {
+            const int m = (k * q) % R;
+            const T c = (T)root_cos<R>(m <= H ? m : R - m);
+            const T s = (T)(m <= H ? root_sin<R>(m) : -root_sin<R>(R - m));
+            A.x += c * v[k].x;
+            A.y += c * v[k].y;
+            B.x += s * v[R - k].x;
+            B.y += s * v[R - k].y;
+        }
+        const CT iB = mk<CT>(-B.y, B.x);  // forward: X_q = A - i B
+        out(q, INV ? cadd(A, iB) : csub(A, iB));
+        out(R - q, INV ? csub(A, iB) : cadd(A, iB));
+    }
+}
+
+// The plain sum, with the roots of the twiddle table, for the FP32 spectrum: its round-off decides
+// when a mixed-precision increment stops gaining and goes on in FP64, so its arithmetic stays as it is.
+template <int R, bool INV, class CT, class Out>
+__device__ __forceinline__ void dft_odd_sum(const CT (&v)[R], const CT* __restrict__ tw, int n, const Out& out) {
+    const int step = n / R;
+#pragma unroll
+    for (int q = 0; q < R; q++) {
+        CT acc = v[0];
+#pragma unroll
+        for (int r = 1; r < R; r++) {
+            CT w = tw[((r * q) % R) * step];
+            if (INV) w.y = -w.y;
+            acc = cadd(acc, cmul(v[r], w));
+        }
+        out(q, acc);
+    }
+}
+
+// Where a transform's first stage reads its elements and its last one puts them: the shared
+// pencils (element e of pencil p at s[e * ES + p]), or a functor over (e, p), which takes the
+// values straight between global memory and the stage's registers.
+struct InShared {};
+struct OutShared {};
+template <class T, class U>
+constexpr bool same_type = false;
+template <class T>
+constexpr bool same_type<T, T> = true;
+
+// One Stockham stage over P pencils of length n; element-major in shared memory:
+// element e of pencil p at s[e*ES + p].
+template <int R, bool INV, int MAXB, class CT, class In, class Out>
+__device__ __forceinline__ void fft_stage(CT* s, int ES, int P, int n, int Ns, const CT* __restrict__ tw, const In& in, const Out& out) {
     const int nb = n / R, total = nb * P;
-    CT v[MAXB][R];
+    constexpr bool sin = same_type<In, InShared>, sout = same_type<Out, OutShared>;
+    auto load = [&](int b, CT (&v)[R]) {
+        const int p = b % P, j = b / P;
 #pragma unroll
-    for (int q = 0; q < MAXB; q++) {
-        const int b = threadIdx.x + q * blockDim.x;
-        if (b < total) {
-            const int p = b % P, j = b / P;
+        for (int r = 0; r < R; r++) {
+            if constexpr (sin) v[r] = s[(j + r * nb) * ES + p];
+            else v[r] = in(j + r * nb, p);
+        }
+    };
+    auto finish = [&](int b, CT (&v)[R]) {
+        const int p = b % P, j = b / P, jm = j % Ns;
+        const int step = jm * (n / (Ns * R));
 #pragma unroll
-            for (int r = 0; r < R; r++) v[q][r] = s[(j + r * nb) * ES + p];
+        for (int r = 1; r < R; r++) {
+            CT w = tw[r * step];
+            if (INV) w.y = -w.y;
+            v[r] = cmul(v[r], w);
+        }
+        const int idxD = (j / Ns) * Ns * R + jm;
+        auto put = [&](int r, CT x) {
+            if constexpr (sout) s[(idxD + r * Ns) * ES + p] = x;
+            else out(idxD + r * Ns, p, x);
+        };
+        if constexpr (R % 2 != 0) {
+            if constexpr (sizeof(CT) == 16) dft_odd<R, INV, CT>(v, put);
+            else dft_odd_sum<R, INV, CT>(v, tw, n, put);
+        } else {
+            dft_small<R, INV, CT>(v);
+#pragma unroll
+            for (int r = 0; r < R; r++) put(r, v[r]);
+        }
+    };
+    if constexpr (sin && sout) {  // in place: every butterfly is read before the first is written
+        CT v[MAXB][R];
+#pragma unroll
+        for (int q = 0; q < MAXB; q++) {
+            const int b = threadIdx.x + q * blockDim.x;
+            if (b < total) load(b, v[q]);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < MAXB; q++) {
+            const int b = threadIdx.x + q * blockDim.x;
+            if (b < total) finish(b, v[q]);
+        }
+    } else {  // one butterfly after the other: half the registers
+#pragma unroll 1
+        for (int b = threadIdx.x; b < total; b += blockDim.x) {
+            CT v[R];
+            load(b, v);
+            finish(b, v);
         }
     }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < MAXB; q++) {
-        const int b = threadIdx.x + q * blockDim.x;
-        if (b < total) {
-            const int p = b % P, j = b / P, jm = j % Ns;
-            const int step = jm * (n / (Ns * R));
-#pragma unroll
-            for (int r = 1; r < R; r++) {
-                CT w = tw[r * step];
-                if (INV) w.y = -w.y;
-                v[q][r] = cmul(v[q][r], w);
-            }
-            dft_small<R, INV, CT>(v[q], tw, n);
-            const int idxD = (j / Ns) * Ns * R + jm;
-#pragma unroll
-            for (int r = 0; r < R; r++) s[(idxD + r * Ns) * ES + p] = v[q][r];
-        }
-    }
-    __syncthreads();
+    if constexpr (sout) __syncthreads();
 }
 
-// Radix sets: RS = 0 compiles the power-of-two radices only (2, 4, 8), RS = 1
-// every radix.  Butterflies per thread fall with the radix so that no stage
-// holds more than 16 complex values per thread: two for every power-of-two
+// Radix sets: RS = 0 compiles the power-of-two radices only (2, 4, 8), RS = 1 adds 3 and 5, RS = 2
+// adds 7, 11 and 13, whose registers every plan of its kernels pays for (50x45x36: y passes 19.8 us in
+// the full set, 13.8 without them, event-timed).  Butterflies per thread fall with the radix so that
+// no stage holds more than 16 complex values per thread: two for every power-of-two
 // radix with RS = 0; four for radices 2-4, two for 5-8 and one for 11 and 13
-// with RS = 1.  Every kernel then fits 128 registers, two blocks of 256
+// otherwise.  Every kernel then fits 128 registers, two blocks of 256
 // threads per SM; the launchers size blocks for the stage that needs the most
 // threads (stage_threads).
 __host__ __device__ constexpr int fft_maxb_r(int rs, int R) { return rs == 0 ? 2 : (R <= 4 ? 4 : (R <= 8 ? 2 : 1)); }
@@ -156,35 +247,76 @@ __host__ __device__ constexpr int fft_maxb_r(int rs, int R) { return rs == 0 ? 2
 // then allocated apart from a kernel with a heavy epilogue (the grid-update z pass).
 template <int R, bool INV, int MAXB, class CT>
 __device__ __noinline__ void fft_stage_call(CT* s, int ES, int P, int n, int Ns, const CT* __restrict__ tw) {
-    fft_stage<R, INV, MAXB, CT>(s, ES, P, n, Ns, tw);
+    fft_stage<R, INV, MAXB, CT>(s, ES, P, n, Ns, tw, InShared{}, OutShared{});
 }
-template <int R, bool INV, int MAXB, class CT, bool CALL>
-__device__ __forceinline__ void fft_stage_odd(CT* s, int ES, int P, int n, int Ns, const CT* __restrict__ tw) {
-    if constexpr (CALL) fft_stage_call<R, INV, MAXB, CT>(s, ES, P, n, Ns, tw);
-    else fft_stage<R, INV, MAXB, CT>(s, ES, P, n, Ns, tw);
+template <int R, bool INV, int RS, class CT, bool CALL, class In, class Out>
+__device__ __forceinline__ void fft_stage_odd(CT* s, int ES, int P, int n, int Ns, const CT* __restrict__ tw, const In& in, const Out& out) {
+    if constexpr (CALL && same_type<In, InShared> && same_type<Out, OutShared>)
+        fft_stage_call<R, INV, fft_maxb_r(RS, R), CT>(s, ES, P, n, Ns, tw);
+    else fft_stage<R, INV, fft_maxb_r(RS, R), CT>(s, ES, P, n, Ns, tw, in, out);
 }
-
-template <bool INV, int RS, class CT, bool ODD_CALL = false>
-__device__ void fft_run(CT* s, int ES, int P, const FftPlan1D& pl, const CT* __restrict__ tw) {
+template <bool INV, int RS, class CT, bool ODD_CALL, class In, class Out>
+__device__ __forceinline__ void fft_stage_any(int R, CT* s, int ES, int P, int n, int Ns, const CT* __restrict__ tw, const In& in, const Out& out) {
+    switch (R) {
+        case 2: fft_stage<2, INV, fft_maxb_r(RS, 2), CT>(s, ES, P, n, Ns, tw, in, out); break;
+        case 4: fft_stage<4, INV, fft_maxb_r(RS, 4), CT>(s, ES, P, n, Ns, tw, in, out); break;
+        case 8: fft_stage<8, INV, fft_maxb_r(RS, 8), CT>(s, ES, P, n, Ns, tw, in, out); break;
+        default:
+            if constexpr (RS != 0) {
+                switch (R) {
+                    case 3: fft_stage_odd<3, INV, RS, CT, ODD_CALL>(s, ES, P, n, Ns, tw, in, out); break;
+                    case 5: fft_stage_odd<5, INV, RS, CT, ODD_CALL>(s, ES, P, n, Ns, tw, in, out); break;
+                    default:
+                        if constexpr (RS == 2) {
+                            switch (R) {
+                                case 7: fft_stage_odd<7, INV, RS, CT, ODD_CALL>(s, ES, P, n, Ns, tw, in, out); break;
+                                case 11: fft_stage_odd<11, INV, RS, CT, ODD_CALL>(s, ES, P, n, Ns, tw, in, out); break;
+                                case 13: fft_stage_odd<13, INV, RS, CT, ODD_CALL>(s, ES, P, n, Ns, tw, in, out); break;
+                                default: break;
+                            }
+                        }
+                        break;
+                }
+            }
+            break;
+    }
+}
+// The whole transform.  With functors at both ends a transform of one stage never touches the
+// shared pencils, one of two stages passes through them once (a plan of no stages, n = 1, copies).
+// The y passes and the outer ends of the z pass use them: staged through shared memory (the y
+// passes by TMA bulk copies) each element crossed it twice more, with a barrier each time.  Event-
+// timed at 64^3 FP64: y 27.6 -> 19.8 us, z with the Green operator 44.5 -> 39; at 128^3 FP32 y
+// 88 -> 47, z 147 -> 123.
+template <bool INV, int RS, class CT, bool ODD_CALL = false, class In = InShared, class Out = OutShared>
+__device__ void fft_run(CT* s, int ES, int P, const FftPlan1D& pl, const CT* __restrict__ tw, const In& in = In{}, const Out& out = Out{}) {
+    constexpr bool gin = !same_type<In, InShared>, gout = !same_type<Out, OutShared>;
+    if constexpr (gin || gout) {
+        if (pl.nst == 0) {
+            for (int p = threadIdx.x; p < P; p += blockDim.x) {
+                CT v;
+                if constexpr (gin) v = in(0, p);
+                else v = s[p];
+                if constexpr (gout) out(0, p, v);
+                else s[p] = v;
+            }
+            __syncthreads();
+            return;
+        }
+        if (gin && gout && pl.nst == 1) {
+            fft_stage_any<INV, RS, CT, ODD_CALL>(pl.rad[0], s, ES, P, pl.n, 1, tw, in, out);
+            return;
+        }
+    }
     int Ns = 1;
+    const int last = pl.nst - 1;
     for (int st = 0; st < pl.nst; st++) {
         const int R = pl.rad[st];
-        switch (R) {
-            case 2: fft_stage<2, INV, fft_maxb_r(RS, 2), CT>(s, ES, P, pl.n, Ns, tw); break;
-            case 4: fft_stage<4, INV, fft_maxb_r(RS, 4), CT>(s, ES, P, pl.n, Ns, tw); break;
-            case 8: fft_stage<8, INV, fft_maxb_r(RS, 8), CT>(s, ES, P, pl.n, Ns, tw); break;
-            default:
-                if constexpr (RS != 0) {
-                    switch (R) {
-                        case 3: fft_stage_odd<3, INV, fft_maxb_r(RS, 3), CT, ODD_CALL>(s, ES, P, pl.n, Ns, tw); break;
-                        case 5: fft_stage_odd<5, INV, fft_maxb_r(RS, 5), CT, ODD_CALL>(s, ES, P, pl.n, Ns, tw); break;
-                        case 7: fft_stage_odd<7, INV, fft_maxb_r(RS, 7), CT, ODD_CALL>(s, ES, P, pl.n, Ns, tw); break;
-                        case 11: fft_stage_odd<11, INV, fft_maxb_r(RS, 11), CT, ODD_CALL>(s, ES, P, pl.n, Ns, tw); break;
-                        case 13: fft_stage_odd<13, INV, fft_maxb_r(RS, 13), CT, ODD_CALL>(s, ES, P, pl.n, Ns, tw); break;
-                        default: break;
-                    }
-                }
-                break;
+        if (gin && st == 0) {
+            if constexpr (gin) fft_stage_any<INV, RS, CT, ODD_CALL>(R, s, ES, P, pl.n, Ns, tw, in, OutShared{});
+        } else if (gout && st == last) {
+            if constexpr (gout) fft_stage_any<INV, RS, CT, ODD_CALL>(R, s, ES, P, pl.n, Ns, tw, InShared{}, out);
+        } else {
+            fft_stage_any<INV, RS, CT, ODD_CALL>(R, s, ES, P, pl.n, Ns, tw, InShared{}, OutShared{});
         }
         Ns *= R;
     }
@@ -308,77 +440,19 @@ __global__ void __launch_bounds__(256, 2) k_fft_x_fwd(Dev d, FftPlan1D pl, int G
 }
 
 // ---------------------------------------------------------------- y (C2C)
-// TMA staging of pencils: nrows rows of ncol FP64 complex values (16 bytes each, so both
-// ends of every row are 16-byte aligned), row r from global src(r) to shared dst(r), by bulk
-// copies that complete on one mbarrier.  Thread 0 posts the expected byte count, then the 32
-// lanes of warp 0 issue the rows; every thread waits for the bytes with a bounded wait (each
-// try_wait suspends for a while before it fails; past the bound the error word gets bit 3 and
-// the solve stops).  Callers zero the columns past the spectrum's edge with ordinary stores.
-template <class SrcF, class DstF>
-__device__ __forceinline__ void tma_rows(int nrows, int ncol, SrcF src, DstF dst, int* err) {
-    __shared__ __align__(8) unsigned long long bar;
-    const unsigned sbar = (unsigned)__cvta_generic_to_shared(&bar);
-    if (threadIdx.x == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sbar) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        if (threadIdx.x == 0) {
-            const unsigned bytes = (unsigned)(nrows * ncol * 16);
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sbar), "r"(bytes) : "memory");
-        }
-        __syncwarp();
-        for (int r = threadIdx.x; r < nrows; r += 32) {
-            const unsigned d = (unsigned)__cvta_generic_to_shared(dst(r));
-            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(d),
-                         "l"(src(r)), "r"((unsigned)(ncol * 16)), "r"(sbar)
-                         : "memory");
-        }
-    }
-    unsigned done = 0;
-    for (long tries = 0; !done; tries++) {
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(done)
-                     : "r"(sbar)
-                     : "memory");
-        if (!done && tries > (1L << 20)) {
-            atomicOr(err, 8);
-            break;
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(sbar) : "memory");
-}
-
 template <bool INV, int RS, class CT>
 __device__ __forceinline__ void body_fft_y(const Dev& d, const FftPlan1D& pl, int T, const VB& vb) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     CT* const s = reinterpret_cast<CT*>(smem_raw);
     const int n1h = d.n1h, n2 = d.n2, n3 = d.n3;
     const int kx0 = vb.x * T, k3 = vb.y, c = vb.z;
-    CT* base = reinterpret_cast<CT*>(d.spec) + ((long long)c * n3 + k3) * n2 * n1h;
-    if constexpr (sizeof(CT) == 16) {
-        // FP64 spectrum: the block's pencils arrive by TMA bulk copies, one per y row (its valid columns)
-        const int ncol = min(T, n1h - kx0);
-        for (int idx = threadIdx.x; idx < (T - ncol) * n2; idx += blockDim.x) {
-            const int t = ncol + idx % (T - ncol), j = idx / (T - ncol);
-            s[j * T + t] = mk<CT>(0, 0);
-        }
-        tma_rows(n2, ncol, [&](int j) { return base + (long long)j * n1h + kx0; }, [&](int j) { return s + (size_t)j * T; },
-                 d.err);
-    } else {
-        for (int idx = threadIdx.x; idx < T * n2; idx += blockDim.x) {
-            const int t = idx % T, j = idx / T, kx = kx0 + t;
-            s[j * T + t] = (kx < n1h) ? base[(long long)j * n1h + kx] : mk<CT>(0, 0);
-        }
-        __syncthreads();
-    }
-    fft_run<INV, RS, CT>(s, T, T, pl, twid<CT>(d, 2));
-    for (int idx = threadIdx.x; idx < T * n2; idx += blockDim.x) {
-        const int t = idx % T, j = idx / T, kx = kx0 + t;
-        if (kx < n1h) base[(long long)j * n1h + kx] = s[j * T + t];
-    }
+    CT* const base = reinterpret_cast<CT*>(d.spec) + ((long long)c * n3 + k3) * n2 * n1h + kx0;
+    const int ncol = min(T, n1h - kx0);
+    fft_run<INV, RS, CT>(
+        s, T, T, pl, twid<CT>(d, 2), [&](int e, int p) { return p < ncol ? base[e * n1h + p] : mk<CT>(0, 0); },
+        [&](int e, int p, CT v) {
+            if (p < ncol) base[e * n1h + p] = v;
+        });
 }
 template <bool INV, int RS, class CT>
 __global__ void __launch_bounds__(256, 2) k_fft_y(Dev d, FftPlan1D pl, int T) { body_fft_y<INV, RS, CT>(d, pl, T, hw_vb()); }
@@ -422,14 +496,13 @@ __device__ __forceinline__ void body_fft_z_green(const Dev& d, const FftPlan1D& 
     const int P = 9 * T;
     for (int i = threadIdx.x; i < 81; i += blockDim.x) { c0[i] = (Re)c0g[i]; s0[i] = (Re)s0g[i]; }
     const long long plane = (long long)n2 * n1h;
-    // ordinary loads: the block's rows are short (T complex values per component and z), which
-    // suits TMA bulk copies badly (measured: 43 -> 68 us per 64^3 launch with one copy per row)
-    for (int idx = threadIdx.x; idx < P * n3; idx += blockDim.x) {
-        const int t = idx % T, r = idx / T, c = r % 9, k3 = r / 9, kx = kx0 + t;
-        s[k3 * P + c * T + t] = (kx < n1h) ? spec[((long long)c * n3 + k3) * plane + (long long)j * n1h + kx] : mk<CT>(0, 0);
-    }
+    CT* const base = spec + (long long)j * n1h + kx0;
+    const int ncol = min(T, n1h - kx0);
     __syncthreads();
-    fft_run<false, RS, CT>(s, P, P, pl, twid<CT>(d, 3));
+    fft_run<false, RS, CT>(s, P, P, pl, twid<CT>(d, 3), [&](int e, int p) {
+        const int c = p / T, t = p - c * T;
+        return t < ncol ? base[((long long)c * n3 + e) * plane + t] : mk<CT>(0, 0);
+    });
     const bool nyq_y = (n2 % 2 == 0 && j == n2 / 2);
     const Re xiy = (Re)xi_of(j, n2);
     for (int idx = threadIdx.x; idx < T * n3; idx += blockDim.x) {
@@ -509,11 +582,10 @@ __device__ __forceinline__ void body_fft_z_green(const Dev& d, const FftPlan1D& 
         for (int c = 0; c < 9; c++) q[c * T] = r[c];
     }
     __syncthreads();
-    fft_run<true, RS, CT>(s, P, P, pl, twid<CT>(d, 3));
-    for (int idx = threadIdx.x; idx < P * n3; idx += blockDim.x) {
-        const int t = idx % T, r = idx / T, c = r % 9, k3 = r / 9, kx = kx0 + t;
-        if (kx < n1h) spec[((long long)c * n3 + k3) * plane + (long long)j * n1h + kx] = s[k3 * P + c * T + t];
-    }
+    fft_run<true, RS, CT>(s, P, P, pl, twid<CT>(d, 3), InShared{}, [&](int e, int p, CT v) {
+        const int c = p / T, t = p - c * T;
+        if (t < ncol) base[((long long)c * n3 + e) * plane + t] = v;
+    });
 }
 template <int RS, class CT>
 __global__ void __launch_bounds__(256, 2) k_fft_z_green(Dev d, FftPlan1D pl, int T, const double* __restrict__ c0g,
@@ -654,22 +726,33 @@ __device__ __forceinline__ void body_fft_x_inv(const Dev& d, const FftPlan1D& pl
     const int P = ncomp * G;
     const int pair0 = vb.x * G;
     const bool even = (n1 % 2 == 0);
-    for (int idx = threadIdx.x; idx < P * n1; idx += blockDim.x) {
-        const int x = idx % n1, p = idx / n1;
-        const int c = p / G, g = p % G;
-        const int ra = 2 * (pair0 + g);
-        const int k = (x <= n1 / 2) ? x : n1 - x;
-        const bool cj = (x > n1 / 2);
-        CT A = mk<CT>(0, 0), B = mk<CT>(0, 0);
-        if (ra < nrows) A = spec[((long long)c * nrows + ra) * n1h + k];
-        if (ra + 1 < nrows) B = spec[((long long)c * nrows + ra + 1) * n1h + k];
-        if (k == 0 || (even && k == n1 / 2)) { A.y = 0; B.y = 0; }
-        if (cj) { A.y = -A.y; B.y = -B.y; }
-        s[x * P + p] = mk<CT>(A.x - B.y, A.y + B.x);
+    // four values of both rows in flight per thread: the compiler keeps global loads behind the
+    // shared-memory stores before them
+    constexpr int U = 4;
+    for (int i0 = threadIdx.x; i0 < P * n1; i0 += U * blockDim.x) {
+        CT A[U], B[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int idx = i0 + u * blockDim.x;
+            const int x = idx % n1, p = idx / n1, c = p / G, ra = 2 * (pair0 + p % G);
+            const int k = (x <= n1 / 2) ? x : n1 - x;
+            const CT* const q = spec + ((long long)c * nrows + ra) * n1h + k;
+            const bool in = idx < P * n1;
+            A[u] = in && ra < nrows ? q[0] : mk<CT>(0, 0);
+            B[u] = in && ra + 1 < nrows ? q[n1h] : mk<CT>(0, 0);
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int idx = i0 + u * blockDim.x;
+            if (idx >= P * n1) break;
+            const int x = idx % n1, p = idx / n1;
+            if (x == 0 || (even && x == n1 / 2)) { A[u].y = 0; B[u].y = 0; }
+            if (x > n1 / 2) { A[u].y = -A[u].y; B[u].y = -B[u].y; }
+            s[x * P + p] = mk<CT>(A[u].x - B[u].y, A[u].y + B[u].x);
+        }
     }
     __syncthreads();
     fft_run<true, RS, CT>(s, P, P, pl, twid<CT>(d, 1));
-    const double invN = 1.0 / (double)N;
     double acc[9];
 #pragma unroll
     for (int c = 0; c < 9; c++) acc[c] = 0.0;
@@ -681,21 +764,21 @@ __device__ __forceinline__ void body_fft_x_inv(const Dev& d, const FftPlan1D& pl
         const Re* sd = reinterpret_cast<const Re*>(s);
         if (mode == 0) {
             double t[9], fi[9], u[9];
+            const double w = d.wgtc[v];
 #pragma unroll
             for (int c = 0; c < 9; c++) {
-                t[c] = (double)sd[2 * (x * P + c * G + g) + half] / (double)N;
-                d.dvr[c * N + v] = t[c];
                 fi[c] = d.Finv[c * N + v];
+                t[c] = (double)sd[2 * (x * P + c * G + g) + half] / (double)N;
             }
+#pragma unroll
+            for (int c = 0; c < 9; c++) d.dvr[c * N + v] = t[c];
             mm3(t, fi, u);
-            const double w = d.wgtc[v];
 #pragma unroll
             for (int c = 0; c < 9; c++) acc[c] += w * u[c];
         } else {
             for (int c = 0; c < ncomp; c++) d.dv3[c * N + v] = (double)sd[2 * (x * P + c * G + g) + half] / (double)N;
         }
     }
-    (void)invN;
     if (mode != 0) return;
     // the last block forms du = (dvelgradavg - <dL_ref F^{-1}>) inv(<F^{-1}>)
     __shared__ double fsum[9];
@@ -785,10 +868,22 @@ __global__ void __launch_bounds__(256, 2) k_green_x_inv(Dev d, FftPlan1D pl, int
 // plan has only radices 2, 4 and 8, asks the kernel for its block-size limit
 // (set by its register use) and shrinks its tile (pencils per block) until
 // the threads fit.
-static bool plan_pow2(const FftPlan1D& pl) {
-    for (int i = 0; i < pl.nst; i++)
-        if (pl.rad[i] != 2 && pl.rad[i] != 4 && pl.rad[i] != 8) return false;
-    return true;
+static int plan_set(const FftPlan1D& pl) {  // the smallest radix set that holds the plan
+    int rs = 0;
+    for (int i = 0; i < pl.nst; i++) {
+        const int R = pl.rad[i];
+        rs = std::max(rs, R > 5 && R != 8 ? 2 : (R == 3 || R == 5 ? 1 : 0));
+    }
+    return rs;
+}
+// f(integral constant RS) for a plan's radix set
+template <class F>
+static auto with_set(int rs, F&& f) {
+    switch (rs) {
+        case 0: return f(std::integral_constant<int, 0>{});
+        case 1: return f(std::integral_constant<int, 1>{});
+        default: return f(std::integral_constant<int, 2>{});
+    }
 }
 static int kernel_max_threads(const void* k) {
     cudaFuncAttributes a{};
@@ -864,8 +959,7 @@ static void green_apply_rs(const Dev& d, const FftPlan1D& pl1, const FftPlan1D& 
 }
 void launch_green_apply(const Dev& d, const FftPlan1D& pl1, const FftPlan1D& pl2, const FftPlan1D& pl3, const double* tau,
                         double* out, const double* c0, const double* s0, cudaStream_t st) {
-    if (plan_pow2(pl1)) green_apply_rs<0>(d, pl1, pl2, pl3, tau, out, c0, s0, st);
-    else green_apply_rs<1>(d, pl1, pl2, pl3, tau, out, c0, s0, st);
+    with_set(plan_set(pl1), [&](auto rs) { green_apply_rs<rs()>(d, pl1, pl2, pl3, tau, out, c0, s0, st); });
 }
 
 // ---------------------------------------------------------------- measured tile choice (autotuner)
@@ -939,8 +1033,9 @@ static void x_fwd_rs(const Dev& d, const FftPlan1D& pl, int mode, int sg_off, cu
 }
 void launch_fft_x_fwd(const Dev& d, const FftPlan1D& pl, int mode, int sg_off, cudaStream_t st, int prec) {
     const bool f32 = prec != 0 && mode == 0;  // the grid-update chain (mode 1) stays FP64
-    if (plan_pow2(pl)) f32 ? x_fwd_rs<0, float2>(d, pl, mode, sg_off, st) : x_fwd_rs<0, double2>(d, pl, mode, sg_off, st);
-    else f32 ? x_fwd_rs<1, float2>(d, pl, mode, sg_off, st) : x_fwd_rs<1, double2>(d, pl, mode, sg_off, st);
+    with_set(plan_set(pl), [&](auto rs) {
+        f32 ? x_fwd_rs<rs(), float2>(d, pl, mode, sg_off, st) : x_fwd_rs<rs(), double2>(d, pl, mode, sg_off, st);
+    });
 }
 
 static int y_tile(const Dev& d) {
@@ -968,8 +1063,9 @@ static void y_rs(const Dev& d, const FftPlan1D& pl, int ncomp, bool inverse, cud
     else k_fft_y<false, RS, CT><<<grid, sh.thr, sh.smem, st>>>(d, pl, sh.tile);
 }
 void launch_fft_y(const Dev& d, const FftPlan1D& pl, int ncomp, bool inverse, cudaStream_t st, int prec) {
-    if (plan_pow2(pl)) prec ? y_rs<0, float2>(d, pl, ncomp, inverse, st) : y_rs<0, double2>(d, pl, ncomp, inverse, st);
-    else prec ? y_rs<1, float2>(d, pl, ncomp, inverse, st) : y_rs<1, double2>(d, pl, ncomp, inverse, st);
+    with_set(plan_set(pl), [&](auto rs) {
+        prec ? y_rs<rs(), float2>(d, pl, ncomp, inverse, st) : y_rs<rs(), double2>(d, pl, ncomp, inverse, st);
+    });
 }
 
 static int z_tile(const Dev& d) {
@@ -995,8 +1091,9 @@ static void z_green_rs(const Dev& d, const FftPlan1D& pl, const double* c0, cons
     k_fft_z_green<RS, CT><<<dim3(sh.gx, sh.gy), sh.thr, sh.smem, st>>>(d, pl, sh.tile, c0, s0);
 }
 void launch_fft_z_green(const Dev& d, const FftPlan1D& pl, const double* c0, const double* s0, cudaStream_t st, int prec) {
-    if (plan_pow2(pl)) prec ? z_green_rs<0, float2>(d, pl, c0, s0, st) : z_green_rs<0, double2>(d, pl, c0, s0, st);
-    else prec ? z_green_rs<1, float2>(d, pl, c0, s0, st) : z_green_rs<1, double2>(d, pl, c0, s0, st);
+    with_set(plan_set(pl), [&](auto rs) {
+        prec ? z_green_rs<rs(), float2>(d, pl, c0, s0, st) : z_green_rs<rs(), double2>(d, pl, c0, s0, st);
+    });
 }
 template <int RS>
 static void z_integ_rs(const Dev& d, const FftPlan1D& pl, int ideriv, cudaStream_t st) {
@@ -1010,8 +1107,7 @@ static void z_integ_rs(const Dev& d, const FftPlan1D& pl, int ideriv, cudaStream
     k_fft_z_integ<RS><<<grid, thr, smem, st>>>(d, pl, T, ideriv);
 }
 void launch_fft_z_integ(const Dev& d, const FftPlan1D& pl, int ideriv, cudaStream_t st) {
-    if (plan_pow2(pl)) z_integ_rs<0>(d, pl, ideriv, st);
-    else z_integ_rs<1>(d, pl, ideriv, st);
+    with_set(plan_set(pl), [&](auto rs) { z_integ_rs<rs()>(d, pl, ideriv, st); });
 }
 
 template <int RS>
@@ -1036,15 +1132,13 @@ static void gradient_rs(const Dev& d, const FftPlan1D& pl1, const FftPlan1D& pl2
     const size_t smem = (size_t)9 * G * d.n1 * sizeof(double2);
     k_green_x_fwd<RS><<<grid, thr, smem, st>>>(d, pl1, G, u9);
     launch_fft_y(d, pl2, 9, false, st, 0);
-    if (plan_pow2(pl3)) z_grad_rs<0>(d, pl3, ideriv, st);
-    else z_grad_rs<1>(d, pl3, ideriv, st);
+    with_set(plan_set(pl3), [&](auto rs) { z_grad_rs<rs()>(d, pl3, ideriv, st); });
     launch_fft_y(d, pl2, 9, true, st, 0);
     k_green_x_inv<RS><<<grid, thr, smem, st>>>(d, pl1, G, out);
 }
 void launch_gradient(const Dev& d, const FftPlan1D& pl1, const FftPlan1D& pl2, const FftPlan1D& pl3, const double* u9,
                      double* out, int ideriv, cudaStream_t st) {
-    if (plan_pow2(pl1)) gradient_rs<0>(d, pl1, pl2, pl3, u9, out, ideriv, st);
-    else gradient_rs<1>(d, pl1, pl2, pl3, u9, out, ideriv, st);
+    with_set(plan_set(pl1), [&](auto rs) { gradient_rs<rs()>(d, pl1, pl2, pl3, u9, out, ideriv, st); });
 }
 template <int RS, class CT>
 static FftShape x_inv_shape(const Dev& d, const FftPlan1D& pl, int ncomp) {
@@ -1065,8 +1159,9 @@ static void x_inv_rs(const Dev& d, const FftPlan1D& pl, int mode, const XinvPara
 }
 void launch_fft_x_inv(const Dev& d, const FftPlan1D& pl, int mode, const XinvParams& p, cudaStream_t st, int prec) {
     const bool f32 = prec != 0 && mode == 0;  // the grid-update chain (mode 1) stays FP64
-    if (plan_pow2(pl)) f32 ? x_inv_rs<0, float2>(d, pl, mode, p, st) : x_inv_rs<0, double2>(d, pl, mode, p, st);
-    else f32 ? x_inv_rs<1, float2>(d, pl, mode, p, st) : x_inv_rs<1, double2>(d, pl, mode, p, st);
+    with_set(plan_set(pl), [&](auto rs) {
+        f32 ? x_inv_rs<rs(), float2>(d, pl, mode, p, st) : x_inv_rs<rs(), double2>(d, pl, mode, p, st);
+    });
 }
 
 // Time every candidate tile of the three tunable passes on this solve's grid (the solve's own
@@ -1101,7 +1196,7 @@ static void autotune_rs(const Dev& d, const FftPlan1D& pl1, const FftPlan1D& pl2
     const int ct = sizeof(CT) == sizeof(float2) ? 1 : 0;
     const int nrows = d.n2 * d.n3, npairs = (nrows + 1) / 2;
     auto pick = [&](int pass, int T0, auto&& fits, auto&& launch) {
-        if (tuned_tile(pass, RS, ct, d) > 0) return;
+        if (plan_set(pass == TUNE_XFWD ? pl1 : (pass == TUNE_Y ? pl2 : pl3)) != RS || tuned_tile(pass, RS, ct, d) > 0) return;
         int best = -1;
         float best_ms = 0.f;
         for (int t : tile_candidates(T0)) {
@@ -1147,17 +1242,11 @@ int fft_autotune(const Dev& d, const FftPlan1D& pl1, const FftPlan1D& pl2, const
     const char* off = getenv("EVP_TUNE");  // EVP_TUNE=0: keep the model's tiles (for comparisons)
     if (off && off[0] == '0') return 0;
     std::vector<std::pair<TuneKey, int>> found;
-    // each pass takes the radix set of its own axis (x forward: axis 1, y: axis 2, z: axis 3); tuning
-    // both sets is cheap and covers whichever each axis needs
-    for (int w = 0; w < (prec ? 2 : 1); w++) {
-        if (w == 0) {
-            autotune_rs<0, double2>(d, pl1, pl2, pl3, c0, s0, st, found);
-            autotune_rs<1, double2>(d, pl1, pl2, pl3, c0, s0, st, found);
-        } else {
-            autotune_rs<0, float2>(d, pl1, pl2, pl3, c0, s0, st, found);
-            autotune_rs<1, float2>(d, pl1, pl2, pl3, c0, s0, st, found);
-        }
-    }
+    for (int rs = 0; rs < 3; rs++)  // each pass is tuned in the radix set of its own axis
+        with_set(rs, [&](auto k) {
+            autotune_rs<k(), double2>(d, pl1, pl2, pl3, c0, s0, st, found);
+            if (prec) autotune_rs<k(), float2>(d, pl1, pl2, pl3, c0, s0, st, found);
+        });
     if (found.empty()) return 0;
     std::lock_guard<std::mutex> lk(g_tune_m);
     std::ofstream f;
@@ -1222,19 +1311,19 @@ template <class CT>
 static void member_fft_ct(const Dev& d, const FftPlan1D& pl1, const FftPlan1D& pl2, const FftPlan1D& pl3, int w,
                           MemberJobs& mj) {
     // the radix set of each pass follows its own axis, as in the single-solve launchers
-    const int rs1 = plan_pow2(pl1) ? 0 : 1, rs2 = plan_pow2(pl2) ? 0 : 1, rs3 = plan_pow2(pl3) ? 0 : 1;
+    const int rs1 = plan_set(pl1), rs2 = plan_set(pl2), rs3 = plan_set(pl3);
     auto put = [&](int k, const FftShape& sh, int rs) {
         mj.job[w][k] = Job{0, 0, sh.gx, sh.gy, sh.gz, sh.tile};
         mj.threads[w][k] = sh.thr;
         mj.smem[w][k] = sh.smem;
-        mj.variant[w][k] = rs | (w << 1);
+        mj.variant[w][k] = rs | (w << 2);
     };
-    put(BK_XFWD, rs1 ? x_fwd_shape<1, CT>(d, pl1) : x_fwd_shape<0, CT>(d, pl1), rs1);
-    const FftShape y = rs2 ? y_shape<1, CT>(d, pl2, 9) : y_shape<0, CT>(d, pl2, 9);
+    put(BK_XFWD, with_set(rs1, [&](auto rs) { return x_fwd_shape<rs(), CT>(d, pl1); }), rs1);
+    const FftShape y = with_set(rs2, [&](auto rs) { return y_shape<rs(), CT>(d, pl2, 9); });
     put(BK_YFWD, y, rs2);
     put(BK_YINV, y, rs2);
-    put(BK_ZGREEN, rs3 ? z_green_shape<1, CT>(d, pl3) : z_green_shape<0, CT>(d, pl3), rs3);
-    put(BK_XINV, rs1 ? x_inv_shape<1, CT>(d, pl1, 9) : x_inv_shape<0, CT>(d, pl1, 9), rs1);
+    put(BK_ZGREEN, with_set(rs3, [&](auto rs) { return z_green_shape<rs(), CT>(d, pl3); }), rs3);
+    put(BK_XINV, with_set(rs1, [&](auto rs) { return x_inv_shape<rs(), CT>(d, pl1, 9); }), rs1);
 }
 
 void member_jobs_fft(const Dev& d, const FftPlan1D& pl1, const FftPlan1D& pl2, const FftPlan1D& pl3, int prec, MemberJobs& mj) {
@@ -1255,12 +1344,9 @@ static void batched_fft_ct(const BatchLaunch& L, const BatchParams& P, cudaStrea
     }
 }
 void launch_batched_fft(const BatchLaunch& L, const BatchParams& P, cudaStream_t st) {
-    switch (L.variant) {
-        case 0: batched_fft_ct<0, double2>(L, P, st); break;
-        case 1: batched_fft_ct<1, double2>(L, P, st); break;
-        case 2: batched_fft_ct<0, float2>(L, P, st); break;
-        default: batched_fft_ct<1, float2>(L, P, st); break;
-    }
+    with_set(L.variant & 3, [&](auto rs) {
+        L.variant >> 2 ? batched_fft_ct<rs(), float2>(L, P, st) : batched_fft_ct<rs(), double2>(L, P, st);
+    });
 }
 
 // Raise the dynamic shared-memory limit of the FFT kernels (once per process).
@@ -1290,6 +1376,7 @@ static void configure_rs() {
 void fft_configure() {
     configure_rs<0>();
     configure_rs<1>();
+    configure_rs<2>();
 }
 
 }  // namespace evp
