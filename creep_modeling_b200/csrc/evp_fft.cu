@@ -712,19 +712,10 @@ __global__ void __launch_bounds__(256, 2) k_fft_z_grad(Dev d, FftPlan1D pl, int 
     }
 }
 
-// ---------------------------------------------------------------- x inverse (C2R)
-template <int RS, class CT>
-__device__ __forceinline__ void body_fft_x_inv(const Dev& d, const FftPlan1D& pl, int G, int ncomp, int mode, const XinvParams& xp,
-                                               const VB& vb) {
-    using Re = typename CxT<CT>::T;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    CT* const s = reinterpret_cast<CT*>(smem_raw);
-    const CT* const spec = reinterpret_cast<const CT*>(d.spec);
-    const int n1 = d.n1, n1h = d.n1h;
-    const long long N = d.N;
-    const int nrows = d.n2 * d.n3;
-    const int P = ncomp * G;
-    const int pair0 = vb.x * G;
+// The packed pencils of the x inverse passes: rows 2 (pair0 + g) and the next of component c as the
+// real and imaginary parts of pencil p = c G + g, each row's full spectrum rebuilt from its half.
+template <class CT>
+__device__ __forceinline__ void load_x_inverse(CT* s, const CT* spec, int P, int G, int pair0, int n1, int n1h, int nrows) {
     const bool even = (n1 % 2 == 0);
     // four values of both rows in flight per thread: the compiler keeps global loads behind the
     // shared-memory stores before them
@@ -751,8 +742,25 @@ __device__ __forceinline__ void body_fft_x_inv(const Dev& d, const FftPlan1D& pl
             s[x * P + p] = mk<CT>(A[u].x - B[u].y, A[u].y + B[u].x);
         }
     }
+}
+
+// ---------------------------------------------------------------- x inverse (C2R)
+template <int RS, class CT>
+__device__ __forceinline__ void body_fft_x_inv(const Dev& d, const FftPlan1D& pl, int G, int ncomp, int mode, const XinvParams& xp,
+                                               const VB& vb) {
+    using Re = typename CxT<CT>::T;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    CT* const s = reinterpret_cast<CT*>(smem_raw);
+    const CT* const spec = reinterpret_cast<const CT*>(d.spec);
+    const int n1 = d.n1, n1h = d.n1h;
+    const long long N = d.N;
+    const int nrows = d.n2 * d.n3;
+    const int P = ncomp * G;
+    const int pair0 = vb.x * G;
+    load_x_inverse(s, spec, P, G, pair0, n1, n1h, nrows);
     __syncthreads();
     fft_run<true, RS, CT>(s, P, P, pl, twid<CT>(d, 1));
+    const double invN = 1.0 / (double)N;
     double acc[9];
 #pragma unroll
     for (int c = 0; c < 9; c++) acc[c] = 0.0;
@@ -768,7 +776,7 @@ __device__ __forceinline__ void body_fft_x_inv(const Dev& d, const FftPlan1D& pl
 #pragma unroll
             for (int c = 0; c < 9; c++) {
                 fi[c] = d.Finv[c * N + v];
-                t[c] = (double)sd[2 * (x * P + c * G + g) + half] / (double)N;
+                t[c] = (double)sd[2 * (x * P + c * G + g) + half] * invN;
             }
 #pragma unroll
             for (int c = 0; c < 9; c++) d.dvr[c * N + v] = t[c];
@@ -776,7 +784,7 @@ __device__ __forceinline__ void body_fft_x_inv(const Dev& d, const FftPlan1D& pl
 #pragma unroll
             for (int c = 0; c < 9; c++) acc[c] += w * u[c];
         } else {
-            for (int c = 0; c < ncomp; c++) d.dv3[c * N + v] = (double)sd[2 * (x * P + c * G + g) + half] / (double)N;
+            for (int c = 0; c < ncomp; c++) d.dv3[c * N + v] = (double)sd[2 * (x * P + c * G + g) + half] * invN;
         }
     }
     if (mode != 0) return;
@@ -836,21 +844,10 @@ __global__ void __launch_bounds__(256, 2) k_green_x_inv(Dev d, FftPlan1D pl, int
     const int nrows = d.n2 * d.n3;
     const int P = 9 * G;
     const int pair0 = blockIdx.x * G;
-    const bool even = (n1 % 2 == 0);
-    for (int idx = threadIdx.x; idx < P * n1; idx += blockDim.x) {
-        const int x = idx % n1, p = idx / n1;
-        const int c = p / G, g = p % G;
-        const int ra = 2 * (pair0 + g);
-        const int k = (x <= n1 / 2) ? x : n1 - x;
-        double2 A = make_double2(0.0, 0.0), B = make_double2(0.0, 0.0);
-        if (ra < nrows) A = d.spec[((long long)c * nrows + ra) * n1h + k];
-        if (ra + 1 < nrows) B = d.spec[((long long)c * nrows + ra + 1) * n1h + k];
-        if (k == 0 || (even && k == n1 / 2)) { A.y = 0.0; B.y = 0.0; }
-        if (x > n1 / 2) { A.y = -A.y; B.y = -B.y; }
-        s[x * P + p] = make_double2(A.x - B.y, A.y + B.x);
-    }
+    load_x_inverse(s, (const double2*)d.spec, P, G, pair0, n1, n1h, nrows);
     __syncthreads();
     fft_run<true, RS, double2>(s, P, P, pl, d.tw1);
+    const double invN = 1.0 / (double)N;
     const double* sd = reinterpret_cast<const double*>(s);
     for (int idx = threadIdx.x; idx < G * 2 * n1; idx += blockDim.x) {
         const int g = idx / (2 * n1), rem = idx % (2 * n1), half = rem / n1, x = rem % n1;
@@ -858,7 +855,7 @@ __global__ void __launch_bounds__(256, 2) k_green_x_inv(Dev d, FftPlan1D pl, int
         if (row >= nrows) continue;
         const long long v = (long long)row * n1 + x;
 #pragma unroll
-        for (int c = 0; c < 9; c++) out[c * N + v] = sd[2 * (x * P + c * G + g) + half] / (double)N;
+        for (int c = 0; c < 9; c++) out[c * N + v] = sd[2 * (x * P + c * G + g) + half] * invN;
     }
 }
 
