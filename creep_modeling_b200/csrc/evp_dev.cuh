@@ -25,6 +25,7 @@ struct PhaseDev {
     double hard[kMaxSysDev * kMaxSysDev];
     double dnca[kMaxSysDev * 3], dbca[kMaxSysDev * 3];
     double C[81];
+    double C66[36];  // C in the b-basis
 };
 
 // One phase as the local solve reads it (NS: 12 or 24 systems), staged into shared memory by a

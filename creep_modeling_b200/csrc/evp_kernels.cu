@@ -571,16 +571,32 @@ __global__ void __launch_bounds__(kBlock) k_upd2(Dev d, Upd2Params p) {
             // (the rotation of the crystal stiffness by aa = Fe ag as two 6x6 products in the
             // b-basis, Q c Q^T with Q = rot_b66(aa), instead of index by index over 3x3x3x3 and
             // chg_basis: the same tensor, rounding apart)
-            double ag[9], aa[9], Q[36], cc[36], c66[36];
+            double ag[9], aa[9], Q[36], c66[21], s66[21];
             ld9(d.ag, N, v, ag);
             mm3(Fe, ag, aa);
-            const double detFe = det33(Fe);
+            const double idet = 1.0 / det33(Fe);
             rot_b66(aa, Q);
-            t4_to_b66(ph.C, cc);
-            congruence6(Q, cc, 1.0 / detFe, c66);
-            if (inv_unrolled<6>(c66) != 0) set_err(d.err, 1);
 #pragma unroll
-            for (int c = 0; c < 36; c++) d.sg66[c * N + v] = c66[c];
+            for (int i = 0; i < 6; i++) {
+                double ta[6];
+#pragma unroll
+                for (int j = 0; j < 6; j++) {
+                    double x = 0.0;
+#pragma unroll
+                    for (int k = 0; k < 6; k++) x += Q[6 * i + k] * ph.C66[6 * k + j];
+                    ta[j] = x;
+                }
+#pragma unroll
+                for (int j = 0; j <= i; j++) {
+                    double x = 0.0;
+#pragma unroll
+                    for (int k = 0; k < 6; k++) x += ta[k] * Q[6 * j + k];
+                    c66[tri(i, j)] = idet * x;
+                }
+            }
+            if (inv_sym6(c66, s66) != 0) set_err(d.err, 1);
+#pragma unroll
+            for (int c = 0; c < 36; c++) d.sg66[c * N + v] = s66[tri(c / 6, c % 6)];
         } else {
             ld9(d.Feinc, N, v, Feinc);
         }
@@ -822,10 +838,12 @@ void launch_diag(const Dev& d, double Lfloor, cudaStream_t st) { k_diag<<<d.grid
 template <int NS>
 __global__ void __launch_bounds__(kC0Block) k_c0(Dev d, double tdot, double tdotref) {
     const long long N = d.N;
-    // each thread's 72 running sums in its own shared-memory slice (registers hold the per-voxel work)
+    // each thread's 42 running sums (the lower triangles of both tangents) in a shared-memory column,
+    // entry c of thread t at [c * kC0Block + t]: conflict free, and registers hold the per-voxel work
     extern __shared__ double c0acc[];
-    double* const s = c0acc + threadIdx.x * 72;
-    for (int c = 0; c < 72; c++) s[c] = 0.0;
+    double* const s = c0acc + threadIdx.x;
+    for (int c = 0; c < 42; c++) s[c * kC0Block] = 0.0;
+    const double itr = 1.0 / tdotref;
     for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < N; v += (long long)gridDim.x * blockDim.x) {
         if (d.gas[v]) continue;
         const PhaseDev& ph = d.ph[d.phase[v]];
@@ -839,31 +857,54 @@ __global__ void __launch_bounds__(kC0Block) k_c0(Dev d, double tdot, double tdot
             tt[q][1] = (q < d.nsys) ? d.trialtau[(2 * q + 1) * N + v] : 1.0;
         }
         constitutive<NS>(ph, d.sch, N, v, tt, sg, ep, dd, gd);
-        double tr[36];
+        // de/dsg = S / tdotref + dd, symmetric positive definite, and its inverse
+        double h[21], tr[21];
 #pragma unroll
         for (int i = 0; i < 6; i++)
 #pragma unroll
-            for (int j = 0; j < 6; j++) tr[6 * i + j] = d.sg66[(6 * i + j) * N + v] / tdot * tdot / tdotref + dd_at(dd, i, j);
-        if (inv_unrolled<6>(tr) != 0) set_err(d.err, 1);
+            for (int j = 0; j <= i; j++) h[tri(i, j)] = d.sg66[(6 * j + i) * N + v] * itr + dd_at(dd, i, j);
+        if (inv_sym6(h, tr) != 0) set_err(d.err, 1);
         // dsg = tr in the b-basis (summed here, expanded to 3x3x3x3 on the host); the PK1 tangent
         // dpg_ijkl = J sum_mn dsg_imkn Fi_jm Fi_ln has the b-basis components J T(Fi) tr T(Fi)^T
-        double Fi[9], T[36], dp6[36];
+        double Fi[9], T[36];
         ld9(d.Finv, N, v, Fi);
         const double detF = d.detF[v], w = d.wgtc[v];
         basis_T(Fi, T);
-        congruence6(T, tr, detF, dp6);
 #pragma unroll
-        for (int c = 0; c < 36; c++) s[c] += tr[c] * w;
+        for (int c = 0; c < 21; c++) s[c * kC0Block] += tr[c] * w;
 #pragma unroll
-        for (int c = 0; c < 36; c++) s[36 + c] += dp6[c] * d.wgt;
+        for (int i = 0; i < 6; i++) {
+            double ta[6];
+#pragma unroll
+            for (int j = 0; j < 6; j++) {
+                double x = 0.0;
+#pragma unroll
+                for (int k = 0; k < 6; k++) x += T[6 * i + k] * tr[tri(k, j)];
+                ta[j] = x;
+            }
+#pragma unroll
+            for (int j = 0; j <= i; j++) {
+                double x = 0.0;
+#pragma unroll
+                for (int k = 0; k < 6; k++) x += ta[k] * T[6 * j + k];
+                s[(21 + tri(i, j)) * kC0Block] += (detF * x) * d.wgt;
+            }
+        }
     }
-    reduce_store<72, 0>(s, nullptr, d.partials, d.red + OFF_C0, d.counters + CNT_C0, hw_vb());
+    __shared__ double fs[42];
+    if (!reduce_store<42, 0>(s, nullptr, d.partials, fs, d.counters + CNT_C0, hw_vb(), kC0Block)) return;
+    __syncthreads();
+    for (int c = threadIdx.x; c < 72; c += blockDim.x) {
+        const int e = c % 36;
+        d.red[OFF_C0 + c] = fs[(c / 36) * 21 + tri(e / 6, e % 6)];
+    }
 }
 void launch_c0(const Dev& d, double tdot, double tdotref, cudaStream_t st) {
-    const size_t sm = (size_t)kC0Block * 72 * sizeof(double);
+    const size_t sm = (size_t)kC0Block * 42 * sizeof(double);
     // four blocks per SM (the 255-register bound allows four of 64 threads): one wave, each
-    // thread several voxels, and a fold of 592 block partials per field instead of 2368
-    // (measured 624 -> 498 us at 64^3)
+    // thread several voxels, and a fold of 592 block partials per field instead of 2368.
+    // At 64^3 (event-timed) 434 us with 72 sums a thread side by side (16-way bank conflicts),
+    // the general inverse and two divisions for each entry of S / tdotref; 142 now.
     const long long g = (d.N + kC0Block - 1) / kC0Block;
     const int grid = (int)(g < 148LL * 4 ? g : 148LL * 4);
     if (d.nsys <= 12) {

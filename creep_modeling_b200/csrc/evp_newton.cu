@@ -251,7 +251,6 @@ struct ColV {
 };
 template <int NS>
 __host__ __device__ constexpr int newtonv_threads_per_sm() { return NS <= 12 ? 256 : 128; }
-__host__ __device__ constexpr int tri(int i, int j) { return i >= j ? i * (i + 1) / 2 + j : j * (j + 1) / 2 + i; }
 
 // Loads and stores of fields that the kernel writes, ordered among themselves and known to be global
 // memory (the compiler would otherwise order every shared-memory access around them).

@@ -482,6 +482,7 @@ public:
                 }
             }
             for (int c = 0; c < 81; c++) t.C[c] = s.C[c];
+            t4_to_b66(t.C, t.C66);
         }
         PhaseDev* dph = dalloc<PhaseDev>(dk.nph);
         h2d_copy(dph, ph.data(), dk.nph * sizeof(PhaseDev));

@@ -47,16 +47,16 @@ __host__ __device__ constexpr int pow2_at_least(int n) { return n <= 1 ? 1 : 2 *
 __host__ __device__ constexpr int log2_of(int n) { return n <= 1 ? 0 : 1 + log2_of(n / 2); }
 // fields [F0, F0 + NF) of the thread's values into sh[f] (one row per warp)
 template <int NF, bool MAX, int F0 = 0>
-__device__ __forceinline__ void warp_fields(const double* vals, double* sh, int lane) {
+__device__ __forceinline__ void warp_fields(const double* vals, double* sh, int lane, int stride = 1) {
     if constexpr (F0 < NF) {
         constexpr int n = NF - F0 < 32 ? NF - F0 : 32, W = pow2_at_least(n);
         double x[W];
 #pragma unroll
-        for (int f = 0; f < W; f++) x[f] = f < n ? vals[F0 + f] : (MAX ? -EVP_HUGE : 0.0);
+        for (int f = 0; f < W; f++) x[f] = f < n ? vals[(F0 + f) * stride] : (MAX ? -EVP_HUGE : 0.0);
         const double y = warp_reduce_many<W, MAX>(x, lane);
         constexpr int sft = 5 - log2_of(W);
         if ((lane & ((1 << sft) - 1)) == 0 && (lane >> sft) < n) sh[F0 + (lane >> sft)] = y;
-        warp_fields<NF, MAX, F0 + 32>(vals, sh, lane);
+        warp_fields<NF, MAX, F0 + 32>(vals, sh, lane, stride);
     }
 }
 // fold of fields f0, f0 + step, f0 + 2 step, f0 + 3 step (below nf) over the block partials by one warp
@@ -95,15 +95,15 @@ __device__ __forceinline__ void fold_four(const double* partials, int nblk, int 
 }
 
 // Returns true in every thread of the block that folded (out is then written, visible to the
-// block after a __syncthreads); blocks of at most 8 warps, whole warps.
+// block after a __syncthreads); blocks of at most 8 warps, whole warps.  stride: between a thread's sums.
 template <int NS, int NM>
 __device__ bool reduce_store(const double* sums, const double* maxs, double* partials, double* out, unsigned int* counter,
-                             const VB& vb) {
+                             const VB& vb, int stride = 1) {
     constexpr int NF = NS + NM;
     __shared__ double sh[8][NF];
     __shared__ bool last;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-    warp_fields<NS, false>(sums, sh[warp], lane);
+    warp_fields<NS, false>(sums, sh[warp], lane, stride);
     warp_fields<NM, true>(maxs, sh[warp] + NS, lane);
     __syncthreads();
     for (int f = threadIdx.x; f < NF; f += blockDim.x) {
@@ -155,6 +155,77 @@ __device__ __forceinline__ double rcp_nr(double x) {
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
     y = fma(y, fma(-x, y, 1.0), y);
     return fma(y, fma(-x, y, 1.0), y);
+}
+
+__host__ __device__ constexpr int tri(int i, int j) { return i >= j ? i * (i + 1) / 2 + j : j * (j + 1) / 2 + i; }
+
+// the general inverse, for a matrix that the symmetric one refuses
+__device__ __noinline__ inline int inv_general6(const double* h21, double* x21) {
+    double J[36];
+#pragma unroll
+    for (int i = 0; i < 6; i++)
+#pragma unroll
+        for (int j = 0; j < 6; j++) J[6 * i + j] = h21[tri(i, j)];
+    const int info = inv_unrolled<6>(J);
+#pragma unroll
+    for (int i = 0; i < 6; i++)
+#pragma unroll
+        for (int j = 0; j <= i; j++) x21[tri(i, j)] = J[6 * i + j];
+    return info;
+}
+// Inverse of a symmetric positive definite 6x6 matrix (packed lower triangles) from its L D L^T
+// factors: M = L^-1, X = M^T D^-1 M, 21 entries instead of 36 and no pivoting.  A pivot that is not
+// positive sends it to the general elimination.  Returns nonzero for a singular matrix.
+__device__ __forceinline__ int inv_sym6(const double (&h)[21], double (&x)[21]) {
+    double a[21], inv[6];
+    bool spd = true;
+#pragma unroll
+    for (int i = 0; i < 21; i++) a[i] = h[i];
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+        spd = spd && a[tri(k, k)] > 0.0;
+        inv[k] = rcp_nr(a[tri(k, k)]);
+        double l[6];
+#pragma unroll
+        for (int i = k + 1; i < 6; i++) l[i] = a[tri(i, k)] * inv[k];
+#pragma unroll
+        for (int i = k + 1; i < 6; i++) {
+#pragma unroll
+            for (int j = k + 1; j <= i; j++) a[tri(i, j)] -= l[i] * a[tri(j, k)];
+        }
+#pragma unroll
+        for (int i = k + 1; i < 6; i++) a[tri(i, k)] = l[i];  // L below the diagonal
+    }
+    if (!spd) {
+        double hh[21], xx[21];
+#pragma unroll
+        for (int i = 0; i < 21; i++) hh[i] = h[i];
+        const int info = inv_general6(hh, xx);
+#pragma unroll
+        for (int i = 0; i < 21; i++) x[i] = xx[i];
+        return info;
+    }
+#pragma unroll
+    for (int j = 0; j < 6; j++)
+#pragma unroll
+        for (int i = j + 1; i < 6; i++) {  // column j of M below the diagonal, in place of L's rows used up
+            double t = a[tri(i, j)];
+#pragma unroll
+            for (int k = j + 1; k < i; k++) t += a[tri(i, k)] * x[tri(k, j)];
+            x[tri(i, j)] = -t;
+        }
+#pragma unroll
+    for (int i = 0; i < 6; i++)
+#pragma unroll
+        for (int j = 0; j <= i; j++) {  // X_ij = sum over k >= i of M_ki M_kj / d_k, rows in rising order
+            double t = i == j ? inv[i] : inv[i] * x[tri(i, j)];
+#pragma unroll
+            for (int k = i + 1; k < 6; k++) t += inv[k] * x[tri(k, i)] * x[tri(k, j)];
+            a[tri(i, j)] = t;
+        }
+#pragma unroll
+    for (int i = 0; i < 21; i++) x[i] = a[i];
+    return 0;
 }
 
 // |x|^e for the power law: integer exponents by binary powering, else pow().
