@@ -32,7 +32,7 @@ struct PhaseDev {
 // straight copy.  Systems beyond the phase's own have n = 1 and gamd0 = 0: they never slip.
 template <int NS>
 struct PhaseV {
-    int nsyst, nmodes, int_exp, kuni;  // kuni: the exponent n - 1 when it is one integer for every system, else -1
+    int nsyst, nmodes, pad0, kuni;  // kuni: the exponent n - 1 when it is one integer for every system, else -1
     int nsm[3], pad;
     double ng[2 * NS];                // gamd0, n of each system
     double hard[NS * NS];             // rows start on 16 bytes
@@ -117,6 +117,7 @@ struct Dev {
                // bit 3 a TMA bulk copy that did not complete within its bounded wait
     const PhaseDev *ph;
     const double* phv;  // the phases as PhaseV<12> (at most 12 systems) or PhaseV<24>
+    int uniexp;         // 1: every solid phase has one integer exponent n - 1 for its systems
     int nph;
 };
 

@@ -236,9 +236,9 @@ __global__ void __launch_bounds__(kNewtonBlock, 2) k_newton(Dev d, NewtonParams 
 // a thread and the 840 B column both allow 256 threads per SM with 12 systems, 128 with 24; the
 // systems of an evaluation give each warp independent work, which replaces occupancy.  Against six
 // lanes per voxel, which exchanged every vector between lanes (243 M warp instructions per launch
-// at 64^3, now 64 M), a launch takes 238 us instead of 621 (64^3, 12 systems, n = 20, 3.0
-// evaluations per voxel; 0.50 GB of DRAM traffic, FP64 pipe 28 % busy), 174 instead of 347 (40^3,
-// 24 systems), 35 instead of 105 (32^3, --modal 1), and the same 30 at 16^3, where each SM has one
+// at 64^3, now 64 M), a launch takes 231 us instead of 621 (64^3, 12 systems, n = 20, 3.0
+// evaluations per voxel; 0.50 GB of DRAM traffic, FP64 pipe 28 % busy), 167 instead of 347 (40^3,
+// 24 systems), 32 instead of 105 (32^3, --modal 1), and 29 instead of 31 at 16^3, where each SM has one
 // warp and its chain is all there is.  32 voxels of a warp wait for the slowest: 84 % of the slots
 // work.  Measured without gain at 64^3: L2 prefetch of the next batch (290 -> 322 us: two batches of
 // 51 kB per warp do not fit the L2), its asynchronous copies issued before this batch's closing sums
@@ -405,7 +405,7 @@ __device__ __forceinline__ void reduce_newton(const double (*sh)[kNewtonSums], d
 
 // Resolved shears over resistance rs and powers |rs|^(n-1) of G systems (Schmid vectors cs,
 // reciprocal resistances ci, (gamd0, n) pairs ng), each step on all of them so that their chains overlap.
-template <int G>
+template <int G, bool UNI>
 __device__ __forceinline__ void slip_powers(const double* cs, const double* ci, const double* ng, int kuni,
                                             const double (&sg)[6], double (&rs)[G], double (&pw)[G]) {
 #pragma unroll
@@ -415,7 +415,7 @@ __device__ __forceinline__ void slip_powers(const double* cs, const double* ci, 
         for (int c = 1; c < 5; c++) x += cs[(5 * q + c) * 32] * sg[c];
         rs[q] = x * ci[2 * q * 32 + (x < 0.0 ? 32 : 0)];
     }
-    if (kuni >= 0) {  // one integer exponent: binary powering of the systems together
+    if (UNI || kuni >= 0) {  // one integer exponent: binary powering of the systems together
         double b[G];
 #pragma unroll
         for (int q = 0; q < G; q++) {
@@ -435,7 +435,9 @@ __device__ __forceinline__ void slip_powers(const double* cs, const double* ci, 
     }
 }
 
-template <int NS>
+// UNI: every phase has one integer exponent for its systems; the kernel then holds no pow(), which
+// would take registers and instruction cache from the common case.
+template <int NS, bool UNI>
 __device__ __forceinline__ void body_newtonv(const Dev& d, const NewtonParams& p, const VB& vb) {
     using Col = ColV<NS>;
     extern __shared__ __align__(16) double dyn_smem[];
@@ -565,11 +567,13 @@ __device__ __forceinline__ void body_newtonv(const Dev& d, const NewtonParams& p
                                 const double* const cs = col + (Col::sch + 5 * s0) * 32;
                                 const double* const ci = col + (Col::itau + 2 * s0) * 32;
                                 double rs[kG], pw[kG];
-                                slip_powers<kG>(cs, ci, &ph.ng[2 * s0], ph.kuni, sg, rs, pw);
+                                slip_powers<kG, UNI>(cs, ci, &ph.ng[2 * s0], ph.kuni, sg, rs, pw);
 #pragma unroll
                                 for (int q = 0; q < kG; q++) {
                                     const double2 ng = *reinterpret_cast<const double2*>(&ph.ng[2 * (s0 + q)]);
                                     const double dum = ng.x * pw[q], g = rs[q] * dum;
+                                    if constexpr (!UNI)
+                                        if (2 * (s0 + q) < qlast) st_rw(d.gamdot + (s0 + q) * N + v, g);
                                     const double r1 = ng.y * dum * ci[2 * q * 32 + (rs[q] < 0.0 ? 32 : 0)];
                                     double sc[5];
 #pragma unroll
@@ -630,10 +634,12 @@ __device__ __forceinline__ void body_newtonv(const Dev& d, const NewtonParams& p
                         }
                         more = sgnorm > 0.0 ? dsg2 > errlim2 : dsg2 > 0.0;
                     }
-                    // the slip rates at the last evaluation's stress, formed again (a third of an evaluation)
-                    // instead of kept in registers or written and read back at each evaluation
+                    // The slip rates at the last evaluation's stress.  With an integer exponent they are formed
+                    // again (a third of an evaluation) instead of kept in registers; where each power is a
+                    // call of pow() the evaluations left them in their output array (50x45x36, n = 12.6:
+                    // 201 -> 180 us per launch).
                     double gd[NS], dg = 0.0;
-                    {
+                    if constexpr (UNI) {
                         double se[6], *out = d.gamdot + v;
 #pragma unroll
                         for (int i = 0; i < 6; i++) se[i] = sgold[i];
@@ -643,18 +649,28 @@ __device__ __forceinline__ void body_newtonv(const Dev& d, const NewtonParams& p
 #pragma unroll
                         for (int s0 = 0; s0 < NS; s0 += kG) {
                             double rs[kG], pw[kG];
-                            slip_powers<kG>(col + (Col::sch + 5 * s0) * 32, col + (Col::itau + 2 * s0) * 32, &ph.ng[2 * s0], ph.kuni, se,
-                                            rs, pw);
+                            slip_powers<kG, UNI>(col + (Col::sch + 5 * s0) * 32, col + (Col::itau + 2 * s0) * 32, &ph.ng[2 * s0], ph.kuni, se,
+                                                  rs, pw);
 #pragma unroll
                             for (int q = 0; q < kG; q++) {
                                 const double g = rs[q] * (ph.ng[2 * (s0 + q)] * pw[q]);
                                 gd[s0 + q] = fabs(g);
-                                dg += fabs(g);
                                 if (2 * (s0 + q) < qlast) st_rw(out, g);
                                 out += N;
                             }
                         }
+                    } else {
+                        const double* q = d.gamdot + v;
+#pragma unroll
+                        for (int s = 0; s < NS; s++) {
+                            gd[s] = ld_rw(q);
+                            q += 2 * s < qlast - 1 ? N : 0;
+                        }
+#pragma unroll
+                        for (int s = 0; s < NS; s++) gd[s] = s < nsyst ? fabs(gd[s]) : 0.0;
                     }
+#pragma unroll
+                    for (int s = 0; s < NS; s++) dg += gd[s];
                     if (!p.iuphard) break;
                     // harden (various_functions.f90:1439-1491).  The new resistances go to their output array;
                     // the old ones, for the norm of the change, are the column's reciprocals inverted.
@@ -778,26 +794,27 @@ __device__ __forceinline__ void body_newtonv(const Dev& d, const NewtonParams& p
     }
     reduce_newton(sh, d.partials, d.red + OFF_NEWTON, d.counters + CNT_NEWTON, vb);
 }
-template <int NS>
-__global__ void __launch_bounds__(newtonv_threads_per_sm<NS>(), 1) k_newtonv(Dev d, NewtonParams p) { body_newtonv<NS>(d, p, hw_vb()); }
+template <int NS, bool UNI>
+__global__ void __launch_bounds__(newtonv_threads_per_sm<NS>(), 1) k_newtonv(Dev d, NewtonParams p) { body_newtonv<NS, UNI>(d, p, hw_vb()); }
 
-// The local-solve kernel of a solve: 0/1 k_newtonv<12/24> (at most kMaxPhaseSmem phases, whose
-// tables fit beside the columns), 6/7 k_newton<12/24>, which reads every operator from memory
-// (more phases, and EVP_NEWTON_ONE_THREAD=1 for comparison).
+// The local-solve kernel of a solve: 0/1 k_newtonv<12/24> for integer exponents, 2/3 for others (at
+// most kMaxPhaseSmem phases, whose tables fit beside the columns), 6/7 k_newton<12/24>, which reads
+// every operator from memory (more phases, and EVP_NEWTON_ONE_THREAD=1 for comparison).
 static int newton_kernel(const Dev& d) {
     static const bool one_thread = [] {
         const char* e = getenv("EVP_NEWTON_ONE_THREAD");
         return e && e[0] == '1';
     }();
     const int big = d.nsys > 12 ? 1 : 0;
-    return (one_thread || d.nph > kMaxPhaseSmem ? 6 : 0) + big;
+    return (one_thread || d.nph > kMaxPhaseSmem ? 6 : (d.uniexp ? 0 : 2)) + big;
 }
+constexpr int newton_sm_threads(int kernel) { return kernel & 1 ? newtonv_threads_per_sm<24>() : newtonv_threads_per_sm<12>(); }
 // Block size of k_newtonv: as many threads as an SM holds (one block per SM, the fewest partial
 // sums to fold) unless that leaves SMs without a block; then halved until every SM has one, down
 // to one warp.
 static int newton_threads(const Dev& d, int kernel) {
     if (kernel >= 6) return kNewtonBlock;
-    int t = kernel == 0 ? newtonv_threads_per_sm<12>() : newtonv_threads_per_sm<24>();
+    int t = newton_sm_threads(kernel);
     while (t > 32 && (d.N + t - 1) / t < 148) t /= 2;
     return t;
 }
@@ -805,29 +822,27 @@ static int newton_grid(const Dev& d, int kernel) {
     const long long t = newton_threads(d, kernel), g = (d.N + t - 1) / t;
     if (kernel >= 6) return (int)(g < 148LL * 16 ? g : 148LL * 16);
     // one wave, every warp taking every (blocks x warps)-th batch of 32 voxels
-    const long long wave = 148LL * ((kernel == 0 ? newtonv_threads_per_sm<12>() : newtonv_threads_per_sm<24>()) / t);
+    const long long wave = 148LL * (newton_sm_threads(kernel) / t);
     return (int)(g < wave ? g : wave);
 }
 static size_t newton_smem(const Dev& d, int kernel) {
     const size_t t = newton_threads(d, kernel);
-    switch (kernel) {
-        case 0: return d.nph * sizeof(PhaseV<12>) + sizeof(double) * ColV<12>::n * t;
-        case 1: return d.nph * sizeof(PhaseV<24>) + sizeof(double) * ColV<24>::n * t;
-        default: return 0;
-    }
+    if (kernel >= 6) return 0;
+    return kernel & 1 ? d.nph * sizeof(PhaseV<24>) + sizeof(double) * ColV<24>::n * t
+                      : d.nph * sizeof(PhaseV<12>) + sizeof(double) * ColV<12>::n * t;
 }
 template <int V>
-constexpr int kb_newton_bound() { return V >= 6 ? kNewtonBlock : (V == 0 ? newtonv_threads_per_sm<12>() : newtonv_threads_per_sm<24>()); }
+constexpr int kb_newton_bound() { return V >= 6 ? kNewtonBlock : newton_sm_threads(V); }
 template <int V>
 __global__ void __launch_bounds__(kb_newton_bound<V>(), V >= 6 ? 2 : 1) kb_newton(const __grid_constant__ BatchParams P);
 static void newton_configure() {
     static std::once_flag once;
     std::call_once(once, [] {
         const int lim = 222 * 1024;
-        cudaFuncSetAttribute(k_newtonv<12>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-        cudaFuncSetAttribute(k_newtonv<24>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-        cudaFuncSetAttribute(kb_newton<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-        cudaFuncSetAttribute(kb_newton<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+        const void* const ks[] = {(const void*)k_newtonv<12, true>, (const void*)k_newtonv<24, true>, (const void*)k_newtonv<12, false>,
+                                  (const void*)k_newtonv<24, false>, (const void*)kb_newton<0>, (const void*)kb_newton<1>,
+                                  (const void*)kb_newton<2>, (const void*)kb_newton<3>};
+        for (const void* k : ks) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
     });
 }
 
@@ -836,8 +851,10 @@ void launch_newton(const Dev& d, const NewtonParams& p, cudaStream_t st) {
     const int k = newton_kernel(d), grid = newton_grid(d, k), thr = newton_threads(d, k);
     const size_t sm = newton_smem(d, k);
     switch (k) {
-        case 0: k_newtonv<12><<<grid, thr, sm, st>>>(d, p); break;
-        case 1: k_newtonv<24><<<grid, thr, sm, st>>>(d, p); break;
+        case 0: k_newtonv<12, true><<<grid, thr, sm, st>>>(d, p); break;
+        case 1: k_newtonv<24, true><<<grid, thr, sm, st>>>(d, p); break;
+        case 2: k_newtonv<12, false><<<grid, thr, sm, st>>>(d, p); break;
+        case 3: k_newtonv<24, false><<<grid, thr, sm, st>>>(d, p); break;
         case 6: k_newton<12><<<grid, thr, 0, st>>>(d, p); break;
         default: k_newton<24><<<grid, thr, 0, st>>>(d, p); break;
     }
@@ -857,8 +874,10 @@ __global__ void __launch_bounds__(kb_newton_bound<V>(), V >= 6 ? 2 : 1) kb_newto
     if (!go) return;
     const NewtonParams p = ps;  // in registers, as a single-solve launch's parameter
     const VB vb = job_vb(jb);
-    if constexpr (V == 0) body_newtonv<12>(m.d, p, vb);
-    else if constexpr (V == 1) body_newtonv<24>(m.d, p, vb);
+    if constexpr (V == 0) body_newtonv<12, true>(m.d, p, vb);
+    else if constexpr (V == 1) body_newtonv<24, true>(m.d, p, vb);
+    else if constexpr (V == 2) body_newtonv<12, false>(m.d, p, vb);
+    else if constexpr (V == 3) body_newtonv<24, false>(m.d, p, vb);
     else if constexpr (V == 6) body_newton1<12>(m.d, p, vb);
     else body_newton1<24>(m.d, p, vb);
 }
@@ -874,6 +893,8 @@ void launch_batched_newton(const BatchLaunch& L, const BatchParams& P, cudaStrea
     switch (L.variant & 7) {
         case 0: kb_newton<0><<<L.blocks, L.threads, L.smem, st>>>(P); break;
         case 1: kb_newton<1><<<L.blocks, L.threads, L.smem, st>>>(P); break;
+        case 2: kb_newton<2><<<L.blocks, L.threads, L.smem, st>>>(P); break;
+        case 3: kb_newton<3><<<L.blocks, L.threads, L.smem, st>>>(P); break;
         case 6: kb_newton<6><<<L.blocks, L.threads, L.smem, st>>>(P); break;
         default: kb_newton<7><<<L.blocks, L.threads, L.smem, st>>>(P); break;
     }

@@ -255,11 +255,12 @@ public:
     template <int NS>
     const double* upload_phases(const std::vector<PhaseDev>& ph) {
         std::vector<PhaseV<NS>> t(ph.size());
+        d.uniexp = 1;
         for (size_t p = 0; p < ph.size(); p++) {
             const PhaseDev& g = ph[p];
             PhaseV<NS>& v = t[p];
             std::memset(&v, 0, sizeof(v));
-            v.nsyst = g.nsyst; v.nmodes = g.nmodes; v.int_exp = g.int_exp;
+            v.nsyst = g.nsyst; v.nmodes = g.nmodes;
             v.kuni = g.int_exp && g.nsyst > 0 ? (int)(g.nrs[0] - 1.0) : -1;
             for (int m = 0; m < 3; m++) {
                 v.nsm[m] = g.nsm[m]; v.tau1[m] = g.tau1[m]; v.thet0[m] = g.thet0[m]; v.thet1[m] = g.thet1[m];
@@ -271,6 +272,7 @@ public:
                 if (own && g.nrs[i] != g.nrs[0]) v.kuni = -1;
                 for (int j = 0; own && j < g.nsyst; j++) v.hard[i * NS + j] = g.hard[i * kMaxSysDev + j];
             }
+            if (!g.igas && v.kuni < 0) d.uniexp = 0;
         }
         double* dst = dalloc<double>(t.size() * sizeof(PhaseV<NS>) / sizeof(double));
         h2d_copy(dst, t.data(), t.size() * sizeof(PhaseV<NS>));
