@@ -47,12 +47,28 @@ Engine::~Engine() {
     if (dE_) cudaFreeAsync(dE_, st_);
     if (dEv_) cudaFreeAsync(dEv_, st_);
     if (hEv_) cudaFreeHost(hEv_);
+    for (int a = 0; a < kAux; a++) {
+        if (aux_[a]) cudaStreamDestroy(aux_[a]);
+        if (join_[a]) cudaEventDestroy(join_[a]);
+    }
+    if (fork_) cudaEventDestroy(fork_);
 }
 
 void Engine::drop_graph() {
     for (auto& g : graphs_)
         if (g) cudaGraphExecDestroy(g);
     graphs_.clear();
+}
+
+void Engine::open_aux() {
+    if (fork_) return;
+    int prio = 0;
+    ECK(cudaStreamGetPriority(st_, &prio));
+    for (int a = 0; a < kAux; a++) {
+        ECK(cudaStreamCreateWithPriority(&aux_[a], cudaStreamNonBlocking, prio));
+        ECK(cudaEventCreateWithFlags(&join_[a], cudaEventDisableTiming));
+    }
+    ECK(cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming));
 }
 
 template <class T>
@@ -138,14 +154,32 @@ void Engine::update_entry(int i, const BatchSolve& e) {
 }
 
 void Engine::launch_one_iteration(const Timer* timer) {
-    for (const Launch& ln : plan_) {
-        if (ln.L.blocks == 0) continue;
-        auto f = [&] {
-            if (fft_kind(ln.L.kind)) launch_batched_fft(ln.L, ln.P, st_);
-            else launch_batched_voxel(ln.L, ln.P, st_);
-        };
-        if (timer) (*timer)(kind_name(ln.L.kind), f);
-        else f();
+    for (size_t i = 0; i < plan_.size();) {
+        size_t e = i;
+        while (e < plan_.size() && plan_[e].L.kind == plan_[i].L.kind) e++;
+        // A pass whose members need several kernels or block sizes: they touch different members, so the
+        // launches run side by side on auxiliary streams (parallel branches of the captured graph).
+        const bool fork = !timer && e - i > 1;
+        const size_t naux = fork ? std::min<size_t>(kAux, e - i - 1) : 0;
+        if (fork) ECK(cudaEventRecord(fork_, st_));
+        for (size_t a = 0; a < naux; a++) ECK(cudaStreamWaitEvent(aux_[a], fork_, 0));
+        for (size_t j = i; j < e; j++) {
+            const Launch& ln = plan_[j];
+            if (ln.L.blocks == 0) continue;
+            const size_t a = j - i;
+            const cudaStream_t st = fork && a > 0 ? aux_[(a - 1) % kAux] : st_;
+            auto f = [&] {
+                if (fft_kind(ln.L.kind)) launch_batched_fft(ln.L, ln.P, st);
+                else launch_batched_voxel(ln.L, ln.P, st);
+            };
+            if (timer) (*timer)(kind_name(ln.L.kind), f);
+            else f();
+        }
+        for (size_t a = 0; a < naux; a++) {
+            ECK(cudaEventRecord(join_[a], aux_[a]));
+            ECK(cudaStreamWaitEvent(st_, join_[a], 0));
+        }
+        i = e;
     }
     auto c = [&] { launch_control(dE_, (int)members_.size(), dEv_, st_); };
     if (timer) (*timer)("k_control", c);
@@ -163,6 +197,7 @@ void Engine::launch(int k, const Timer* timer) {
     cudaGraphExec_t& graph_ = graphs_[k];
     if (!graph_) {
         cudaGraph_t g = nullptr;
+        open_aux();  // not inside the capture
         ECK(cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal));
         for (int i = 0; i < k; i++) launch_one_iteration(nullptr);
         const cudaError_t e1 = cudaGetLastError();

@@ -64,6 +64,7 @@ public:
 
 private:
     void launch_one_iteration(const Timer* timer);
+    void open_aux();  // the auxiliary streams and their events, at the first capture
     void drop_graph();
     template <class T>
     T* grow(T* p, size_t& cap, size_t n);
@@ -74,6 +75,9 @@ private:
         std::vector<int> members;  // their indices in the membership
     };
     cudaStream_t st_;
+    static constexpr int kAux = 4;
+    cudaStream_t aux_[kAux] = {};
+    cudaEvent_t join_[kAux] = {}, fork_ = nullptr;
     std::vector<Member> members_;
     std::vector<Launch> plan_;
     BatchSolve* dE_ = nullptr;  // every member's descriptor, for k_control
