@@ -197,7 +197,8 @@ void Engine::launch(int k, const Timer* timer) {
     cudaGraphExec_t& graph_ = graphs_[k];
     if (!graph_) {
         cudaGraph_t g = nullptr;
-        open_aux();  // not inside the capture
+        for (size_t i = 1; i < plan_.size(); i++)
+            if (plan_[i].L.kind == plan_[i - 1].L.kind) open_aux();  // not inside the capture
         ECK(cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal));
         for (int i = 0; i < k; i++) launch_one_iteration(nullptr);
         const cudaError_t e1 = cudaGetLastError();

@@ -171,7 +171,7 @@ public:
         if (h_red) cudaFreeHost(h_red);
         if (h_err) cudaFreeHost(h_err);
         if (h_ctl) cudaFreeHost(h_ctl);
-        if (h_stage) cudaFreeHost(h_stage);
+        drop_stage();
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
         if (st && own_stream) cudaStreamDestroy(st);
@@ -292,7 +292,6 @@ public:
         if (*h_err & 1) throw SolveError("singular matrix in a voxel operator (lu_inverse / lu_eqsystem)", -3);
         if (*h_err & 2) throw SolveError("non-finite stress in the local Newton solve", -4);
         if (*h_err & 4) throw SolveError("form_G failed (singular acoustic tensor or complex D operator)", -3);
-        if (*h_err & 8) throw SolveError("a bulk copy into shared memory did not complete", -6);
     }
     void fetch_red() {
         fetch_red_async();
@@ -735,7 +734,6 @@ public:
         if (bits & 4) return "form_G failed (singular acoustic tensor or complex D operator)";
         if (bits & 8) return "ERRE/ERRS negative -> convergence failed!";
         if (bits & 32) return "equilibrium iteration did not converge";
-        if (bits & 64) return "a bulk copy into shared memory did not complete";
         return "equilibrium iteration failed";
     }
 
@@ -1345,8 +1343,31 @@ public:
     // the destination's pages overlap (the stress of 128^3, 151 MB: 12 ms; with one pageable copy, a
     // transposition on the host and a second copy in the caller an increment that reads it took 183 ms, now 96).
     static constexpr int kCopiers = 6;
-    static constexpr size_t kPiece = 1 << 18;  // doubles
-    double* h_stage = nullptr;                 // kCopiers pieces, made at the first large field
+    static constexpr size_t kPiece = 1 << 17;  // doubles
+    // The pinned pieces (6 MB) are shared by the solves of the process, one copy at a time, made by the
+    // first solve that reads a large field and given back with the last of those solves: pinning them
+    // for each solve (and the engine's auxiliary streams, now made only for plans that fork) put the
+    // first four increments of a new 64^3 solve at 49 ms, 33 now.
+    struct Stage {
+        std::mutex use, count;
+        double* p = nullptr;
+        int solves = 0;
+    };
+    static Stage& stage() {
+        static Stage s;
+        return s;
+    }
+    bool has_stage = false;
+    void drop_stage() {
+        if (!has_stage) return;
+        Stage& g = stage();
+        std::lock_guard<std::mutex> u(g.use), c(g.count);
+        if (--g.solves == 0) {
+            cudaFreeHost(g.p);
+            g.p = nullptr;
+        }
+        has_stage = false;
+    }
     void to_host(double* dst, const double* src, size_t n) {
         d2h += (long long)(n * sizeof(double));
         if (n < 2 * kPiece) {
@@ -1354,7 +1375,15 @@ public:
             sync();
             return;
         }
-        if (!h_stage) CK(cudaMallocHost(&h_stage, kCopiers * kPiece * sizeof(double)));
+        Stage& g = stage();
+        std::lock_guard<std::mutex> u(g.use);
+        {
+            std::lock_guard<std::mutex> c(g.count);
+            if (!g.p) CK(cudaHostAlloc(&g.p, kCopiers * kPiece * sizeof(double), cudaHostAllocPortable));
+            if (!has_stage) g.solves++;
+            has_stage = true;
+        }
+        double* const h_stage = g.p;
         sync();  // the source is complete
         int dev = 0;
         CK(cudaGetDevice(&dev));

@@ -279,13 +279,6 @@ __device__ __forceinline__ void constitutive(const PhaseDev& ph, const double* _
         }
     }
 }
-// x[i] for a run-time i in 0..5 without a local-memory array
-__device__ __forceinline__ double sel6(const double (&x)[6], int i) {
-    double y = x[0];
-#pragma unroll
-    for (int c = 1; c < 6; c++) y = (i == c) ? x[c] : y;
-    return y;
-}
 __device__ __forceinline__ double dd_at(const double (&dd)[15], int i, int j) {
     if (i > 4 || j > 4) return 0.0;
     int a = i < j ? i : j, b = i < j ? j : i;
