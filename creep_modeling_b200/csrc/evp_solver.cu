@@ -1370,18 +1370,25 @@ public:
     }
     void to_host(double* dst, const double* src, size_t n) {
         d2h += (long long)(n * sizeof(double));
-        if (n < 2 * kPiece) {
+        Stage& g = stage();
+        std::unique_lock<std::mutex> u(g.use, std::defer_lock);
+        bool pieces = n >= 2 * kPiece;
+        if (pieces) {
+            u.lock();
+            std::lock_guard<std::mutex> c(g.count);
+            if (!g.p && cudaHostAlloc(&g.p, kCopiers * kPiece * sizeof(double), cudaHostAllocPortable) != cudaSuccess) {
+                cudaGetLastError();  // no pinned memory to be had: one pageable copy
+                g.p = nullptr;
+                pieces = false;
+            } else {
+                if (!has_stage) g.solves++;
+                has_stage = true;
+            }
+        }
+        if (!pieces) {
             CK(cudaMemcpyAsync(dst, src, n * sizeof(double), cudaMemcpyDeviceToHost, st));
             sync();
             return;
-        }
-        Stage& g = stage();
-        std::lock_guard<std::mutex> u(g.use);
-        {
-            std::lock_guard<std::mutex> c(g.count);
-            if (!g.p) CK(cudaHostAlloc(&g.p, kCopiers * kPiece * sizeof(double), cudaHostAllocPortable));
-            if (!has_stage) g.solves++;
-            has_stage = true;
         }
         double* const h_stage = g.p;
         sync();  // the source is complete
@@ -1794,6 +1801,8 @@ int evp_get_field(evp_solve* h, const char* name, double* host_out, long long ca
         if (written) *written = n;
     } catch (SolveError& e) {
         return fail(e.what(), e.code);
+    } catch (std::exception& e) {  // a copying thread that could not start
+        return fail(e.what(), -6);
     }
     return 0;
 }
