@@ -117,6 +117,7 @@ struct Dev {
     const PhaseDev *ph;
     const double* phv;  // the phases as PhaseV<12> (at most 12 systems) or PhaseV<24>
     int uniexp;         // 1: every solid phase has one integer exponent n - 1 for its systems
+    int symel;          // 1: every phase's stiffness is symmetric (a file may give any 6x6 matrix)
     int nph;
 };
 

@@ -534,6 +534,8 @@ void launch_upd1(const Dev& d, const Upd1Params& p, cudaStream_t st) {
 }
 
 // ---------------------------------------------------------------- k_upd2
+// SYM: every phase's stiffness is symmetric, so its rotation and inverse are formed in 21 entries.
+template <bool SYM>
 __global__ void __launch_bounds__(kBlock) k_upd2(Dev d, Upd2Params p) {
     const long long N = d.N;
     const double dav = __ldcg(&d.red[OFF_UPD1 + 38]);
@@ -571,32 +573,41 @@ __global__ void __launch_bounds__(kBlock) k_upd2(Dev d, Upd2Params p) {
             // (the rotation of the crystal stiffness by aa = Fe ag as two 6x6 products in the
             // b-basis, Q c Q^T with Q = rot_b66(aa), instead of index by index over 3x3x3x3 and
             // chg_basis: the same tensor, rounding apart)
-            double ag[9], aa[9], Q[36], c66[21], s66[21];
+            double ag[9], aa[9], Q[36];
             ld9(d.ag, N, v, ag);
             mm3(Fe, ag, aa);
             const double idet = 1.0 / det33(Fe);
             rot_b66(aa, Q);
+            if constexpr (SYM) {
+                double c66[21], s66[21];
 #pragma unroll
-            for (int i = 0; i < 6; i++) {
-                double ta[6];
+                for (int i = 0; i < 6; i++) {
+                    double ta[6];
 #pragma unroll
-                for (int j = 0; j < 6; j++) {
-                    double x = 0.0;
+                    for (int j = 0; j < 6; j++) {
+                        double x = 0.0;
 #pragma unroll
-                    for (int k = 0; k < 6; k++) x += Q[6 * i + k] * ph.C66[6 * k + j];
-                    ta[j] = x;
+                        for (int k = 0; k < 6; k++) x += Q[6 * i + k] * ph.C66[6 * k + j];
+                        ta[j] = x;
+                    }
+#pragma unroll
+                    for (int j = 0; j <= i; j++) {
+                        double x = 0.0;
+#pragma unroll
+                        for (int k = 0; k < 6; k++) x += ta[k] * Q[6 * j + k];
+                        c66[tri(i, j)] = idet * x;
+                    }
                 }
+                if (inv_sym6(c66, s66) != 0) set_err(d.err, 1);
 #pragma unroll
-                for (int j = 0; j <= i; j++) {
-                    double x = 0.0;
+                for (int c = 0; c < 36; c++) d.sg66[c * N + v] = s66[tri(c / 6, c % 6)];
+            } else {
+                double c66[36];
+                congruence6(Q, ph.C66, idet, c66);
+                if (inv_unrolled<6>(c66) != 0) set_err(d.err, 1);
 #pragma unroll
-                    for (int k = 0; k < 6; k++) x += ta[k] * Q[6 * j + k];
-                    c66[tri(i, j)] = idet * x;
-                }
+                for (int c = 0; c < 36; c++) d.sg66[c * N + v] = c66[c];
             }
-            if (inv_sym6(c66, s66) != 0) set_err(d.err, 1);
-#pragma unroll
-            for (int c = 0; c < 36; c++) d.sg66[c * N + v] = s66[tri(c / 6, c % 6)];
         } else {
             ld9(d.Feinc, N, v, Feinc);
         }
@@ -647,7 +658,10 @@ __global__ void __launch_bounds__(kBlock) k_upd2(Dev d, Upd2Params p) {
         for (int f = 0; f < 9; f++) d.red[OFF_DU2 + f] = du[f];
     }
 }
-void launch_upd2(const Dev& d, const Upd2Params& p, cudaStream_t st) { k_upd2<<<d.grid, d.block, 0, st>>>(d, p); }
+void launch_upd2(const Dev& d, const Upd2Params& p, cudaStream_t st) {
+    if (d.symel) k_upd2<true><<<d.grid, d.block, 0, st>>>(d, p);
+    else k_upd2<false><<<d.grid, d.block, 0, st>>>(d, p);
+}
 
 // ---------------------------------------------------------------- k_upd3
 template <int NS>
@@ -835,14 +849,17 @@ __global__ void __launch_bounds__(kBlock, 2) k_diag(Dev d, double Lfloor) {
 void launch_diag(const Dev& d, double Lfloor, cudaStream_t st) { k_diag<<<d.grid, d.block, 0, st>>>(d, Lfloor); }
 
 // ---------------------------------------------------------------- k_c0
-template <int NS>
+// SYM: every phase's stiffness is symmetric, and with it both tangents.
+__host__ __device__ constexpr int c0_sums(bool sym) { return sym ? 42 : 72; }
+template <int NS, bool SYM>
 __global__ void __launch_bounds__(kC0Block) k_c0(Dev d, double tdot, double tdotref) {
     const long long N = d.N;
-    // each thread's 42 running sums (the lower triangles of both tangents) in a shared-memory column,
+    // each thread's running sums (both tangents, their lower triangles if SYM) in a shared-memory column,
     // entry c of thread t at [c * kC0Block + t]: conflict free, and registers hold the per-voxel work
+    constexpr int kSums = c0_sums(SYM);
     extern __shared__ double c0acc[];
     double* const s = c0acc + threadIdx.x;
-    for (int c = 0; c < 42; c++) s[c * kC0Block] = 0.0;
+    for (int c = 0; c < kSums; c++) s[c * kC0Block] = 0.0;
     const double itr = 1.0 / tdotref;
     for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < N; v += (long long)gridDim.x * blockDim.x) {
         if (d.gas[v]) continue;
@@ -857,63 +874,81 @@ __global__ void __launch_bounds__(kC0Block) k_c0(Dev d, double tdot, double tdot
             tt[q][1] = (q < d.nsys) ? d.trialtau[(2 * q + 1) * N + v] : 1.0;
         }
         constitutive<NS>(ph, d.sch, N, v, tt, sg, ep, dd, gd);
-        // de/dsg = S / tdotref + dd, symmetric positive definite, and its inverse
-        double h[21], tr[21];
-#pragma unroll
-        for (int i = 0; i < 6; i++)
-#pragma unroll
-            for (int j = 0; j <= i; j++) h[tri(i, j)] = d.sg66[(6 * j + i) * N + v] * itr + dd_at(dd, i, j);
-        if (inv_sym6(h, tr) != 0) set_err(d.err, 1);
-        // dsg = tr in the b-basis (summed here, expanded to 3x3x3x3 on the host); the PK1 tangent
-        // dpg_ijkl = J sum_mn dsg_imkn Fi_jm Fi_ln has the b-basis components J T(Fi) tr T(Fi)^T
+        // de/dsg = S / tdotref + dd (symmetric positive definite if SYM) and its inverse dsg in the b-basis
+        // (summed here, expanded to 3x3x3x3 on the host); the PK1 tangent dpg_ijkl = J sum_mn dsg_imkn Fi_jm
+        // Fi_ln has the b-basis components J T(Fi) dsg T(Fi)^T
         double Fi[9], T[36];
-        ld9(d.Finv, N, v, Fi);
-        const double detF = d.detF[v], w = d.wgtc[v];
-        basis_T(Fi, T);
+        if constexpr (SYM) {
+            double h[21], tr[21];
 #pragma unroll
-        for (int c = 0; c < 21; c++) s[c * kC0Block] += tr[c] * w;
+            for (int i = 0; i < 6; i++)
 #pragma unroll
-        for (int i = 0; i < 6; i++) {
-            double ta[6];
+                for (int j = 0; j <= i; j++) h[tri(i, j)] = d.sg66[(6 * j + i) * N + v] * itr + dd_at(dd, i, j);
+            if (inv_sym6(h, tr) != 0) set_err(d.err, 1);
+            ld9(d.Finv, N, v, Fi);
+            const double detF = d.detF[v], w = d.wgtc[v];
+            basis_T(Fi, T);
 #pragma unroll
-            for (int j = 0; j < 6; j++) {
-                double x = 0.0;
+            for (int c = 0; c < 21; c++) s[c * kC0Block] += tr[c] * w;
 #pragma unroll
-                for (int k = 0; k < 6; k++) x += T[6 * i + k] * tr[tri(k, j)];
-                ta[j] = x;
+            for (int i = 0; i < 6; i++) {
+                double ta[6];
+#pragma unroll
+                for (int j = 0; j < 6; j++) {
+                    double x = 0.0;
+#pragma unroll
+                    for (int k = 0; k < 6; k++) x += T[6 * i + k] * tr[tri(k, j)];
+                    ta[j] = x;
+                }
+#pragma unroll
+                for (int j = 0; j <= i; j++) {
+                    double x = 0.0;
+#pragma unroll
+                    for (int k = 0; k < 6; k++) x += ta[k] * T[6 * j + k];
+                    s[(21 + tri(i, j)) * kC0Block] += (detF * x) * d.wgt;
+                }
             }
+        } else {
+            double tr[36], dp6[36];
 #pragma unroll
-            for (int j = 0; j <= i; j++) {
-                double x = 0.0;
+            for (int i = 0; i < 6; i++)
 #pragma unroll
-                for (int k = 0; k < 6; k++) x += ta[k] * T[6 * j + k];
-                s[(21 + tri(i, j)) * kC0Block] += (detF * x) * d.wgt;
+                for (int j = 0; j < 6; j++) tr[6 * i + j] = d.sg66[(6 * i + j) * N + v] * itr + dd_at(dd, i, j);
+            if (inv_unrolled<6>(tr) != 0) set_err(d.err, 1);
+            ld9(d.Finv, N, v, Fi);
+            const double detF = d.detF[v], w = d.wgtc[v];
+            basis_T(Fi, T);
+            congruence6(T, tr, detF, dp6);
+#pragma unroll
+            for (int c = 0; c < 36; c++) {
+                s[c * kC0Block] += tr[c] * w;
+                s[(36 + c) * kC0Block] += dp6[c] * d.wgt;
             }
         }
     }
-    __shared__ double fs[42];
-    if (!reduce_store<42, 0>(s, nullptr, d.partials, fs, d.counters + CNT_C0, hw_vb(), kC0Block)) return;
+    __shared__ double fs[kSums];
+    if (!reduce_store<kSums, 0>(s, nullptr, d.partials, fs, d.counters + CNT_C0, hw_vb(), kC0Block)) return;
     __syncthreads();
     for (int c = threadIdx.x; c < 72; c += blockDim.x) {
         const int e = c % 36;
-        d.red[OFF_C0 + c] = fs[(c / 36) * 21 + tri(e / 6, e % 6)];
+        d.red[OFF_C0 + c] = SYM ? fs[(c / 36) * 21 + tri(e / 6, e % 6)] : fs[c];
     }
 }
+template <int NS, bool SYM>
+static void c0_launch(const Dev& d, int grid, double tdot, double tdotref, cudaStream_t st) {
+    const size_t sm = (size_t)kC0Block * c0_sums(SYM) * sizeof(double);
+    cudaFuncSetAttribute(k_c0<NS, SYM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    k_c0<NS, SYM><<<grid, kC0Block, sm, st>>>(d, tdot, tdotref);
+}
 void launch_c0(const Dev& d, double tdot, double tdotref, cudaStream_t st) {
-    const size_t sm = (size_t)kC0Block * 42 * sizeof(double);
     // four blocks per SM (the 255-register bound allows four of 64 threads): one wave, each
     // thread several voxels, and a fold of 592 block partials per field instead of 2368.
     // At 64^3 (event-timed) 434 us with 72 sums a thread side by side (16-way bank conflicts),
     // the general inverse and two divisions for each entry of S / tdotref; 142 now.
     const long long g = (d.N + kC0Block - 1) / kC0Block;
     const int grid = (int)(g < 148LL * 4 ? g : 148LL * 4);
-    if (d.nsys <= 12) {
-        cudaFuncSetAttribute(k_c0<12>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        k_c0<12><<<grid, kC0Block, sm, st>>>(d, tdot, tdotref);
-    } else {
-        cudaFuncSetAttribute(k_c0<24>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        k_c0<24><<<grid, kC0Block, sm, st>>>(d, tdot, tdotref);
-    }
+    if (d.symel) d.nsys <= 12 ? c0_launch<12, true>(d, grid, tdot, tdotref, st) : c0_launch<24, true>(d, grid, tdot, tdotref, st);
+    else d.nsys <= 12 ? c0_launch<12, false>(d, grid, tdot, tdotref, st) : c0_launch<24, false>(d, grid, tdot, tdotref, st);
 }
 
 // ---------------------------------------------------------------- k_kinematic

@@ -243,14 +243,19 @@ __global__ void __launch_bounds__(kNewtonBlock, 2) k_newton(Dev d, NewtonParams 
 // work.  Measured without gain at 64^3: L2 prefetch of the next batch (290 -> 322 us: two batches of
 // 51 kB per warp do not fit the L2), its asynchronous copies issued before this batch's closing sums
 // (240 -> 243), 12 systems per step (242 -> 324: spills), C~ loaded ahead of the systems (268).
+//
+// SYM false: a phase whose stiffness was given as an asymmetric matrix.  C~, S, G and H are then asymmetric
+// too; every operator is taken with its 36 entries and H goes to the pivoted elimination.  The wider column
+// leaves room for 128 threads per SM: 485 us at 64^3 (630 with six lanes per voxel, 1600 with every operator
+// re-read from memory), 231 at 40^3 with 24 systems (365), 42 at 16^3 (36).
 constexpr int kMaxPhaseSmem = 4;
-// column entries of a thread: Schmid vectors, 1 / resistance (forward, backward), H0 (packed lower triangle)
-template <int NS>
+// column entries of a thread: Schmid vectors, 1 / resistance (forward, backward), H0 (packed lower triangle, or all of it)
+template <int NS, bool SYM>
 struct ColV {
-    static constexpr int sch = 0, itau = 5 * NS, h0 = 7 * NS, n = 7 * NS + 21;
+    static constexpr int sch = 0, itau = 5 * NS, h0 = 7 * NS, n = 7 * NS + (SYM ? 21 : 36);
 };
-template <int NS>
-__host__ __device__ constexpr int newtonv_threads_per_sm() { return NS <= 12 ? 256 : 128; }
+template <int NS, bool SYM>
+__host__ __device__ constexpr int newtonv_threads_per_sm() { return NS <= 12 && SYM ? 256 : 128; }
 
 // Loads and stores of fields that the kernel writes, ordered among themselves and known to be global
 // memory (the compiler would otherwise order every shared-memory access around them).
@@ -334,6 +339,39 @@ __device__ __forceinline__ void ld_sym6(const double* __restrict__ A, long long 
 #pragma unroll
         for (int j = 0; j <= i; j++) a[tri(i, j)] = __ldg(A + (6 * j + i) * N + v);
 }
+// an operator: packed and symmetric, or all of its rows
+template <bool SYM>
+struct Op6 {
+    static constexpr int n = SYM ? 21 : 36;
+    static __host__ __device__ constexpr int at(int i, int j) { return SYM ? tri(i, j) : 6 * i + j; }
+    static __host__ __device__ constexpr int plane(int i, int j) { return SYM ? 6 * j + i : 6 * i + j; }  // entry (i, j <= i if SYM)
+    static __host__ __device__ constexpr int cols(int i) { return SYM ? i + 1 : 6; }  // stored entries of row i
+    static __device__ __forceinline__ void load(const double* __restrict__ A, long long N, long long v, double (&a)[n]) {
+        if constexpr (SYM) {
+            ld_sym6(A, N, v, a);
+        } else {
+#pragma unroll
+            for (int c = 0; c < 36; c++) a[c] = __ldg(A + c * N + v);
+        }
+    }
+    static __device__ __forceinline__ void mv(const double (&A)[n], const double (&x)[6], double (&y)[6]) {
+        if constexpr (SYM) {
+            sym6_mv(A, x, y);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 6; i++) {
+                double t = 0.0;
+#pragma unroll
+                for (int j = 0; j < 6; j++) t += A[6 * i + j] * x[j];
+                y[i] = t;
+            }
+        }
+    }
+    static __device__ __forceinline__ int solve(double (&h)[n], double (&b)[6]) {
+        if constexpr (SYM) return solve_sym6(h, b);
+        else return solve6(h, b);
+    }
+};
 template <int M>
 __device__ __forceinline__ void ldg_n(const double* __restrict__ a, long long N, long long v, double* o) {
 #pragma unroll
@@ -437,9 +475,10 @@ __device__ __forceinline__ void slip_powers(const double* cs, const double* ci, 
 
 // UNI: every phase has one integer exponent for its systems; the kernel then holds no pow(), which
 // would take registers and instruction cache from the common case.
-template <int NS, bool UNI>
+template <int NS, bool UNI, bool SYM>
 __device__ __forceinline__ void body_newtonv(const Dev& d, const NewtonParams& p, const VB& vb) {
-    using Col = ColV<NS>;
+    using Col = ColV<NS, SYM>;
+    using Op = Op6<SYM>;
     extern __shared__ __align__(16) double dyn_smem[];
     PhaseV<NS>* const sph = reinterpret_cast<PhaseV<NS>*>(dyn_smem);
     const int nph = d.nph;  // at most kMaxPhaseSmem (newton_kernel)
@@ -468,7 +507,7 @@ __device__ __forceinline__ void body_newtonv(const Dev& d, const NewtonParams& p
             const PhaseV<NS>& ph = sph[__ldg(d.phase + v)];
             // The batch's inputs are all in flight together: the resistances, B and the Schmid vectors go
             // to the column by asynchronous copies (no registers wait for them), the rest to registers.
-            double l6[6], t6[6], vg[9], e9[9], sm[21], a[9];
+            double l6[6], t6[6], vg[9], e9[9], sm[Op::n], a[9];
             {
                 const double* q = d.trialtau + v;
 #pragma unroll
@@ -480,7 +519,7 @@ __device__ __forceinline__ void body_newtonv(const Dev& d, const NewtonParams& p
 #pragma unroll
                 for (int i = 0; i < 6; i++)
 #pragma unroll
-                    for (int j = 0; j <= i; j++) cp_async8(col + (Col::h0 + tri(i, j)) * 32, q + (6 * j + i) * N);
+                    for (int j = 0; j < Op::cols(i); j++) cp_async8(col + (Col::h0 + Op::at(i, j)) * 32, q + Op::plane(i, j) * N);
                 q = d.sch + v;
 #pragma unroll 10
                 for (int i = 0; i < 5 * NS; i++) {
@@ -488,7 +527,7 @@ __device__ __forceinline__ void body_newtonv(const Dev& d, const NewtonParams& p
                     q += i < slast ? N : 0;
                 }
             }
-            ld_sym6(d.sg66, N, v, sm);
+            Op::load(d.sg66, N, v, sm);
 #pragma unroll
             for (int c = 0; c < 6; c++) l6[c] = ld_rw(d.sg + c * N + v);
             ldg_n<6>(d.sgt, N, v, t6);
@@ -519,11 +558,11 @@ __device__ __forceinline__ void body_newtonv(const Dev& d, const NewtonParams& p
 #pragma unroll
                     for (int i = 0; i < 6; i++)
 #pragma unroll
-                        for (int j = 0; j <= i; j++) {
-                            const double bi = col[(Col::h0 + tri(i, j)) * 32], si = sm[tri(i, j)] * idt;
-                            col[(Col::h0 + tri(i, j)) * 32] = bi + si;
+                        for (int j = 0; j < Op::cols(i); j++) {
+                            const double bi = col[(Col::h0 + Op::at(i, j)) * 32], si = sm[Op::at(i, j)] * idt;
+                            col[(Col::h0 + Op::at(i, j)) * 32] = bi + si;
                             qp[i] += bi * sg[j] + si * sgt[j];
-                            if (j != i) qp[j] += bi * sg[i] + si * sgt[i];
+                            if (SYM && j != i) qp[j] += bi * sg[i] + si * sgt[i];
                         }
 #pragma unroll
                     for (int q = 0; q < 2 * NS; q++) {
@@ -593,14 +632,14 @@ __device__ __forceinline__ void body_newtonv(const Dev& d, const NewtonParams& p
 #pragma unroll
                             for (int i = 0; i < 6; i++)
 #pragma unroll
-                                for (int j = 0; j <= i; j++) {
-                                    const double h = col[(Col::h0 + tri(i, j)) * 32];
+                                for (int j = 0; j < Op::cols(i); j++) {
+                                    const double h = col[(Col::h0 + Op::at(i, j)) * 32];
                                     rho[i] += h * sg[j];
-                                    if (j != i) rho[j] += h * sg[i];
+                                    if (SYM && j != i) rho[j] += h * sg[i];
                                 }
-                            double rn[6], cm[21];
-                            ld_sym6(d.c066mod, N, v, cm);
-                            sym6_mv(cm, rho, rn);
+                            double rn[6], cm[Op::n];
+                            Op::load(d.c066mod, N, v, cm);
+                            Op::mv(cm, rho, rn);
                             res2 = (rn[0] * rn[0] + rn[1] * rn[1]) + (rn[2] * rn[2] + rn[3] * rn[3]) + (rn[4] * rn[4] + rn[5] * rn[5]);
                             if (iterNR == 0) resold2 = res2;
                             halved = false;
@@ -619,13 +658,13 @@ __device__ __forceinline__ void body_newtonv(const Dev& d, const NewtonParams& p
                             c_nr++;
                             if (lane == __ffs(__activemask()) - 1) c_npass++;
                         }
-                        double h[21], dsg2 = 0.0;
+                        double h[Op::n], dsg2 = 0.0;
 #pragma unroll
                         for (int i = 0; i < 6; i++)
 #pragma unroll
-                            for (int j = 0; j <= i; j++)
-                                h[tri(i, j)] = col[(Col::h0 + tri(i, j)) * 32] + (i < 5 ? dd[i < 5 ? tri(i, j) : 0] : 0.0);
-                        if (solve_sym6(h, rho) != 0) set_err(d.err, 1);
+                            for (int j = 0; j < Op::cols(i); j++)
+                                h[Op::at(i, j)] = col[(Col::h0 + Op::at(i, j)) * 32] + dd_at(dd, i, j);
+                        if (Op::solve(h, rho) != 0) set_err(d.err, 1);
 #pragma unroll
                         for (int i = 0; i < 6; i++) {
                             sgold[i] = sg[i];
@@ -734,7 +773,7 @@ __device__ __forceinline__ void body_newtonv(const Dev& d, const NewtonParams& p
                 // |sg - lam|^2 at the final stress; |edot - D|^2 at the last evaluation, with
                 // edot = edotp + S (sg - sgt) / dt + eth as elastic_strain_rate forms it
                 double x6[6], e6[6], D[6], e6v[6], dsg = 0.0, ddg = 0.0;
-                ld_sym6(d.sg66, N, v, sm);
+                Op::load(d.sg66, N, v, sm);
                 ldg_n<6>(d.sgt, N, v, t6);
                 ldg_n<9>(d.velgrad, N, v, vg);
                 if (p.thermo) ldg_n<9>(d.eth, N, v, e9);
@@ -746,7 +785,7 @@ __device__ __forceinline__ void body_newtonv(const Dev& d, const NewtonParams& p
                 s6_to_b6(t6, x6);
 #pragma unroll
                 for (int i = 0; i < 6; i++) x6[i] = (sgold[i] - x6[i]) * idt;
-                sym6_mv(sm, x6, e6);
+                Op::mv(sm, x6, e6);
                 sym33(vg, a);
                 t2_to_b6(a, D);
                 if (p.thermo) t2_to_b6(e9, a);
@@ -794,21 +833,24 @@ __device__ __forceinline__ void body_newtonv(const Dev& d, const NewtonParams& p
     }
     reduce_newton(sh, d.partials, d.red + OFF_NEWTON, d.counters + CNT_NEWTON, vb);
 }
-template <int NS, bool UNI>
-__global__ void __launch_bounds__(newtonv_threads_per_sm<NS>(), 1) k_newtonv(Dev d, NewtonParams p) { body_newtonv<NS, UNI>(d, p, hw_vb()); }
+template <int NS, bool UNI, bool SYM>
+__global__ void __launch_bounds__(newtonv_threads_per_sm<NS, SYM>(), 1) k_newtonv(Dev d, NewtonParams p) { body_newtonv<NS, UNI, SYM>(d, p, hw_vb()); }
 
-// The local-solve kernel of a solve: 0/1 k_newtonv<12/24> for integer exponents, 2/3 for others (at
-// most kMaxPhaseSmem phases, whose tables fit beside the columns), 6/7 k_newton<12/24>, which reads
-// every operator from memory (more phases, and EVP_NEWTON_ONE_THREAD=1 for comparison).
+// The local-solve kernel of a solve: 0/1 k_newtonv<12/24> for integer exponents, 2/3 for others, 4/5 for
+// any with a phase of asymmetric stiffness (at most kMaxPhaseSmem phases, whose tables fit beside the
+// columns), 6/7 k_newton<12/24>, which reads every operator from memory (more phases, and
+// EVP_NEWTON_ONE_THREAD=1 for comparison).
 static int newton_kernel(const Dev& d) {
     static const bool one_thread = [] {
         const char* e = getenv("EVP_NEWTON_ONE_THREAD");
         return e && e[0] == '1';
     }();
     const int big = d.nsys > 12 ? 1 : 0;
-    return (one_thread || d.nph > kMaxPhaseSmem ? 6 : (d.uniexp ? 0 : 2)) + big;
+    return (one_thread || d.nph > kMaxPhaseSmem ? 6 : (!d.symel ? 4 : (d.uniexp ? 0 : 2))) + big;
 }
-constexpr int newton_sm_threads(int kernel) { return kernel & 1 ? newtonv_threads_per_sm<24>() : newtonv_threads_per_sm<12>(); }
+constexpr int newton_sm_threads(int kernel) {
+    return kernel >= 4 ? newtonv_threads_per_sm<12, false>() : (kernel & 1 ? newtonv_threads_per_sm<24, true>() : newtonv_threads_per_sm<12, true>());
+}
 // Block size of k_newtonv: as many threads as an SM holds (one block per SM, the fewest partial
 // sums to fold) unless that leaves SMs without a block; then halved until every SM has one, down
 // to one warp.
@@ -828,8 +870,8 @@ static int newton_grid(const Dev& d, int kernel) {
 static size_t newton_smem(const Dev& d, int kernel) {
     const size_t t = newton_threads(d, kernel);
     if (kernel >= 6) return 0;
-    return kernel & 1 ? d.nph * sizeof(PhaseV<24>) + sizeof(double) * ColV<24>::n * t
-                      : d.nph * sizeof(PhaseV<12>) + sizeof(double) * ColV<12>::n * t;
+    const size_t entries = kernel >= 4 ? (kernel & 1 ? ColV<24, false>::n : ColV<12, false>::n) : (kernel & 1 ? ColV<24, true>::n : ColV<12, true>::n);
+    return d.nph * (kernel & 1 ? sizeof(PhaseV<24>) : sizeof(PhaseV<12>)) + sizeof(double) * entries * t;
 }
 template <int V>
 constexpr int kb_newton_bound() { return V >= 6 ? kNewtonBlock : newton_sm_threads(V); }
@@ -839,9 +881,11 @@ static void newton_configure() {
     static std::once_flag once;
     std::call_once(once, [] {
         const int lim = 222 * 1024;
-        const void* const ks[] = {(const void*)k_newtonv<12, true>, (const void*)k_newtonv<24, true>, (const void*)k_newtonv<12, false>,
-                                  (const void*)k_newtonv<24, false>, (const void*)kb_newton<0>, (const void*)kb_newton<1>,
-                                  (const void*)kb_newton<2>, (const void*)kb_newton<3>};
+        const void* const ks[] = {(const void*)k_newtonv<12, true, true>, (const void*)k_newtonv<24, true, true>,
+                                  (const void*)k_newtonv<12, false, true>, (const void*)k_newtonv<24, false, true>,
+                                  (const void*)k_newtonv<12, false, false>, (const void*)k_newtonv<24, false, false>,
+                                  (const void*)kb_newton<0>, (const void*)kb_newton<1>, (const void*)kb_newton<2>,
+                                  (const void*)kb_newton<3>, (const void*)kb_newton<4>, (const void*)kb_newton<5>};
         for (const void* k : ks) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
     });
 }
@@ -851,10 +895,12 @@ void launch_newton(const Dev& d, const NewtonParams& p, cudaStream_t st) {
     const int k = newton_kernel(d), grid = newton_grid(d, k), thr = newton_threads(d, k);
     const size_t sm = newton_smem(d, k);
     switch (k) {
-        case 0: k_newtonv<12, true><<<grid, thr, sm, st>>>(d, p); break;
-        case 1: k_newtonv<24, true><<<grid, thr, sm, st>>>(d, p); break;
-        case 2: k_newtonv<12, false><<<grid, thr, sm, st>>>(d, p); break;
-        case 3: k_newtonv<24, false><<<grid, thr, sm, st>>>(d, p); break;
+        case 0: k_newtonv<12, true, true><<<grid, thr, sm, st>>>(d, p); break;
+        case 1: k_newtonv<24, true, true><<<grid, thr, sm, st>>>(d, p); break;
+        case 2: k_newtonv<12, false, true><<<grid, thr, sm, st>>>(d, p); break;
+        case 3: k_newtonv<24, false, true><<<grid, thr, sm, st>>>(d, p); break;
+        case 4: k_newtonv<12, false, false><<<grid, thr, sm, st>>>(d, p); break;
+        case 5: k_newtonv<24, false, false><<<grid, thr, sm, st>>>(d, p); break;
         case 6: k_newton<12><<<grid, thr, 0, st>>>(d, p); break;
         default: k_newton<24><<<grid, thr, 0, st>>>(d, p); break;
     }
@@ -874,10 +920,12 @@ __global__ void __launch_bounds__(kb_newton_bound<V>(), V >= 6 ? 2 : 1) kb_newto
     if (!go) return;
     const NewtonParams p = ps;  // in registers, as a single-solve launch's parameter
     const VB vb = job_vb(jb);
-    if constexpr (V == 0) body_newtonv<12, true>(m.d, p, vb);
-    else if constexpr (V == 1) body_newtonv<24, true>(m.d, p, vb);
-    else if constexpr (V == 2) body_newtonv<12, false>(m.d, p, vb);
-    else if constexpr (V == 3) body_newtonv<24, false>(m.d, p, vb);
+    if constexpr (V == 0) body_newtonv<12, true, true>(m.d, p, vb);
+    else if constexpr (V == 1) body_newtonv<24, true, true>(m.d, p, vb);
+    else if constexpr (V == 2) body_newtonv<12, false, true>(m.d, p, vb);
+    else if constexpr (V == 3) body_newtonv<24, false, true>(m.d, p, vb);
+    else if constexpr (V == 4) body_newtonv<12, false, false>(m.d, p, vb);
+    else if constexpr (V == 5) body_newtonv<24, false, false>(m.d, p, vb);
     else if constexpr (V == 6) body_newton1<12>(m.d, p, vb);
     else body_newton1<24>(m.d, p, vb);
 }
@@ -895,6 +943,8 @@ void launch_batched_newton(const BatchLaunch& L, const BatchParams& P, cudaStrea
         case 1: kb_newton<1><<<L.blocks, L.threads, L.smem, st>>>(P); break;
         case 2: kb_newton<2><<<L.blocks, L.threads, L.smem, st>>>(P); break;
         case 3: kb_newton<3><<<L.blocks, L.threads, L.smem, st>>>(P); break;
+        case 4: kb_newton<4><<<L.blocks, L.threads, L.smem, st>>>(P); break;
+        case 5: kb_newton<5><<<L.blocks, L.threads, L.smem, st>>>(P); break;
         case 6: kb_newton<6><<<L.blocks, L.threads, L.smem, st>>>(P); break;
         default: kb_newton<7><<<L.blocks, L.threads, L.smem, st>>>(P); break;
     }

@@ -458,6 +458,7 @@ public:
         }
         // phases
         std::vector<PhaseDev> ph(dk.nph);
+        d.symel = 1;
         for (int p = 0; p < dk.nph; p++) {
             const PhaseData& s = dk.phase[p];
             PhaseDev& t = ph[p];
@@ -482,7 +483,10 @@ public:
                     if (!(e >= 0.0 && e <= 64.0 && e == std::floor(e))) t.int_exp = 0;
                 }
             }
-            for (int c = 0; c < 81; c++) t.C[c] = s.C[c];
+            for (int c = 0; c < 81; c++) {
+                t.C[c] = s.C[c];
+                if (s.C[c] != s.C[9 * (c % 9) + c / 9]) d.symel = 0;  // C_ijkl and C_klij
+            }
             t4_to_b66(t.C, t.C66);
         }
         PhaseDev* dph = dalloc<PhaseDev>(dk.nph);
