@@ -138,6 +138,7 @@ public:
     double last_results[51] = {}, last_diag[44] = {};
     std::vector<double> snap_dsim, snap_scau;
     bool has_thermo = false;
+    size_t spec_size = 0;  // complex values that d.spec holds
     std::vector<double> eth_soa;  // host staging of the thermal eigenstrain upload (kept until the copy completes)
     // optional wall-clock budget: the solve ends with -8 at the first equilibrium iteration after it
     bool has_deadline = false;
@@ -402,7 +403,9 @@ public:
         d.gas = dalloc<uint8_t>(N); d.phase = dalloc<uint8_t>(N);
         d.s_velgrad = dalloc<double>(9 * N); d.s_velgradold = dalloc<double>(9 * N); d.s_sg = dalloc<double>(6 * N);
         d.s_edotp = dalloc<double>(6 * N); d.s_gamdot = dalloc<double>((size_t)ns * N); d.s_trialtau = dalloc<double>(2 * (size_t)ns * N);
-        d.spec = dalloc<double2>(9 * (size_t)d.n1h * dk.n2 * dk.n3);
+        // the spectrum; read-outs interleave fields in it, so it holds at least one voxel's longest record
+        spec_size = std::max<size_t>(9 * (size_t)d.n1h * dk.n2 * dk.n3, kMaxInterleave / 2);
+        d.spec = dalloc<double2>(spec_size);
         {
             bool any_tab = false;
             for (auto& p : dk.process) any_tab = any_tab || p.igamma != 0;
@@ -1428,7 +1431,7 @@ public:
             if (total > cap) return -total - 16;
             if (total == 0) return 0;
             // interleaved on the device, in the spectrum's memory (free between increments), then copied
-            const long long room = 18LL * d.n1h * d.n2 * d.n3 / nout;
+            const long long room = 2 * (long long)spec_size / nout;
             for (long long v0 = 0; v0 < N; v0 += room) {
                 const long long nv = std::min(room, N - v0);
                 launch_interleave(d, dp, map, nout, v0, nv, (double*)d.spec, st);
