@@ -39,6 +39,43 @@ static int check_args(const double* d_tau, double* d_out, int n1, int n2, int n3
     return 0;
 }
 
+// One application on scratch that the entry provides: ntail values (twiddles, c0 and s0, the error word) go
+// behind the spectrum in one upload, then the passes, then the error word back.  Returns the status with its message
+// set; whatever happens, nothing queued here is still running and no exception leaves.
+static int run_green(const std::string& who, Dev& d, const FftPlan1D& pl1, const FftPlan1D& pl2, const FftPlan1D& pl3, double2* dtw,
+                     const double2* tail, size_t ntail, const double* d_tau, double* d_out, cudaStream_t st) {
+    const size_t ntw = (size_t)d.n1 + d.n2 + d.n3;
+    double* const cs = reinterpret_cast<double*>(dtw + ntw);
+    int* const err = reinterpret_cast<int*>(dtw + ntw + 81);
+    d.tw1 = dtw; d.tw2 = dtw + d.n1; d.tw3 = dtw + d.n1 + d.n2;
+    d.err = err;
+    cudaGetLastError();  // an error that the caller has not fetched is not this call's
+    int rc = 0, herr = 0;
+    cudaError_t ce = cudaMemcpyAsync(dtw, tail, ntail * sizeof(double2), cudaMemcpyHostToDevice, st);
+    if (ce == cudaSuccess) {
+        try {
+            launch_green_apply(d, pl1, pl2, pl3, d_tau, d_out, cs, cs + 81, st);
+        } catch (std::exception& e) {  // a length whose pencils fit no block
+            set_last_error(who + ": " + e.what());
+            rc = -2;
+        }
+        ce = cudaGetLastError();  // of the launches
+    }
+    if (ce == cudaSuccess && rc == 0) ce = cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, st);
+    const cudaError_t se = cudaStreamSynchronize(st);
+    if (rc != 0) return rc;
+    if (ce == cudaSuccess) ce = se;
+    if (ce != cudaSuccess) {
+        set_last_error(who + ": " + cudaGetErrorString(ce));
+        return -6;
+    }
+    if (herr) {
+        set_last_error(who + ": singular acoustic tensor");
+        return -3;
+    }
+    return 0;
+}
+
 }  // namespace evp
 
 extern "C" int evp_green_apply(const double* d_tau, double* d_out, int n1, int n2, int n3, const double* c0, const double* s0,
@@ -66,19 +103,11 @@ extern "C" int evp_green_apply(const double* d_tau, double* d_out, int n1, int n
     constexpr size_t kPoolMost = (size_t)1 << 30;
     const size_t nspec = 9 * (size_t)d.n1h * n2 * n3, ntw = (size_t)n1 + n2 + n3, ntail = ntw + 81 + 1;
     const size_t bytes = (nspec + ntail) * sizeof(double2);
-    std::vector<double2> tail(ntail);
-    host_twiddles(n1, tail.data());
-    host_twiddles(n2, tail.data() + n1);
-    host_twiddles(n3, tail.data() + n1 + n2);
-    double* const hcs = reinterpret_cast<double*>(tail.data() + ntw);
-    for (int i = 0; i < 81; i++) {
-        hcs[i] = c0[i];
-        hcs[81 + i] = s0[i];
-    }
-    tail[ntw + 81] = make_double2(0.0, 0.0);  // the error word
+    std::vector<double2> tail;
     const bool pooled = bytes <= kPoolMost;
     void* mem = nullptr;
     try {
+        tail.resize(ntail);
         const cudaError_t ae = pooled ? cudaMallocFromPoolAsync(&mem, bytes, solver_pool(), st) : cudaMalloc(&mem, bytes);
         if (ae != cudaSuccess) {
             cudaGetLastError();
@@ -89,28 +118,20 @@ extern "C" int evp_green_apply(const double* d_tau, double* d_out, int n1, int n
         set_last_error(e.what());
         return -6;
     }
+    host_twiddles(n1, tail.data());
+    host_twiddles(n2, tail.data() + n1);
+    host_twiddles(n3, tail.data() + n1 + n2);
+    double* const hcs = reinterpret_cast<double*>(tail.data() + ntw);
+    for (int i = 0; i < 81; i++) {
+        hcs[i] = c0[i];
+        hcs[81 + i] = s0[i];
+    }
+    tail[ntw + 81] = make_double2(0.0, 0.0);  // the error word
     d.spec = static_cast<double2*>(mem);
-    double2* const dtw = d.spec + nspec;
-    double* const cs = reinterpret_cast<double*>(dtw + ntw);
-    int* const err = reinterpret_cast<int*>(dtw + ntw + 81);
-    d.tw1 = dtw; d.tw2 = dtw + n1; d.tw3 = dtw + n1 + n2;
-    d.err = err;
-    cudaMemcpyAsync(dtw, tail.data(), ntail * sizeof(double2), cudaMemcpyHostToDevice, st);
-    launch_green_apply(d, pl1, pl2, pl3, d_tau, d_out, cs, cs + 81, st);
-    int herr = 0;
-    cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, st);
+    rc = run_green("evp_green_apply", d, pl1, pl2, pl3, d.spec + nspec, tail.data(), ntail, d_tau, d_out, st);
     if (pooled) cudaFreeAsync(mem, st);
-    const cudaError_t ce = cudaStreamSynchronize(st);
-    if (!pooled) cudaFree(mem);
-    if (ce != cudaSuccess) {
-        set_last_error(std::string("evp_green_apply: ") + cudaGetErrorString(ce));
-        return -6;
-    }
-    if (herr) {
-        set_last_error("evp_green_apply: singular acoustic tensor");
-        return -3;
-    }
-    return 0;
+    else cudaFree(mem);
+    return rc;
 }
 
 // ---------------------------------------------------------------- allocation-free variant
@@ -196,31 +217,10 @@ extern "C" int evp_green_apply_noalloc(const double* d_tau, double* d_out, int n
     double* const hcs = reinterpret_cast<double*>(tail + ntw);
     for (int i = 0; i < 81; i++) { hcs[i] = c0[i]; hcs[81 + i] = s0[i]; }
     tail[ntw + 81] = make_double2(0.0, 0.0);
-    double2* const dtw = base + kNoAllocTw;
-    double* const dcs = reinterpret_cast<double*>(dtw + ntw);
-    int* const derr = reinterpret_cast<int*>(dtw + ntw + 81);
-    if (cudaMemcpyAsync(dtw, tail, (ntw + 82) * sizeof(double2), cudaMemcpyHostToDevice, st) != cudaSuccess) {
-        set_last_error("evp_green_apply_noalloc: copy to the scratch failed");
-        return -6;
-    }
     Dev d{};
     d.n1 = n1; d.n2 = n2; d.n3 = n3;
     d.n1h = n1 / 2 + 1;
     d.N = (long long)n1 * n2 * n3;
     d.spec = base;
-    d.tw1 = dtw; d.tw2 = dtw + n1; d.tw3 = dtw + n1 + n2;
-    d.err = derr;
-    launch_green_apply(d, pl1, pl2, pl3, d_tau, d_out, dcs, dcs + 81, st);
-    int herr = 0;
-    cudaMemcpyAsync(&herr, derr, sizeof(int), cudaMemcpyDeviceToHost, st);
-    cudaError_t ce = cudaStreamSynchronize(st);
-    if (ce != cudaSuccess) {
-        set_last_error(std::string("evp_green_apply_noalloc: ") + cudaGetErrorString(ce));
-        return -6;
-    }
-    if (herr) {
-        set_last_error("evp_green_apply_noalloc: singular acoustic tensor");
-        return -3;
-    }
-    return 0;
+    return run_green("evp_green_apply_noalloc", d, pl1, pl2, pl3, base + kNoAllocTw, tail, ntw + 82, d_tau, d_out, st);
 }
