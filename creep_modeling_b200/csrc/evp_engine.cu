@@ -64,9 +64,9 @@ void Engine::open_aux() {
     if (fork_) return;
     int prio = 0;
     ECK(cudaStreamGetPriority(st_, &prio));
-    for (int a = 0; a < kAux; a++) {
-        ECK(cudaStreamCreateWithPriority(&aux_[a], cudaStreamNonBlocking, prio));
-        ECK(cudaEventCreateWithFlags(&join_[a], cudaEventDisableTiming));
+    for (int a = 0; a < kAux; a++) {  // those that an earlier, failed call made are kept
+        if (!aux_[a]) ECK(cudaStreamCreateWithPriority(&aux_[a], cudaStreamNonBlocking, prio));
+        if (!join_[a]) ECK(cudaEventCreateWithFlags(&join_[a], cudaEventDisableTiming));
     }
     ECK(cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming));
 }
@@ -157,8 +157,11 @@ void Engine::launch_one_iteration(const Timer* timer) {
     for (size_t i = 0; i < plan_.size();) {
         size_t e = i;
         while (e < plan_.size() && plan_[e].L.kind == plan_[i].L.kind) e++;
-        // A pass whose members need several kernels or block sizes: they touch different members, so the
-        // launches run side by side on auxiliary streams (parallel branches of the captured graph).
+        // A pass whose members need several kernels, block sizes or precisions: its launches run side by side
+        // on auxiliary streams (parallel branches of the captured graph).  No two of them work on one
+        // member's arrays: each member is in one launch of a pass per spectral precision, and of its FP64 and
+        // FP32 launches one exits at once (batch_go), by ctl->prec, which changes only in k_control, after
+        // the join, and between graph launches.
         const bool fork = !timer && e - i > 1;
         const size_t naux = fork ? std::min<size_t>(kAux, e - i - 1) : 0;
         if (fork) ECK(cudaEventRecord(fork_, st_));
@@ -200,7 +203,14 @@ void Engine::launch(int k, const Timer* timer) {
         for (size_t i = 1; i < plan_.size(); i++)
             if (plan_[i].L.kind == plan_[i - 1].L.kind) open_aux();  // not inside the capture
         ECK(cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal));
-        for (int i = 0; i < k; i++) launch_one_iteration(nullptr);
+        try {
+            for (int i = 0; i < k; i++) launch_one_iteration(nullptr);
+        } catch (...) {  // the stream (and those forked from it) must leave capture mode
+            cudaStreamEndCapture(st_, &g);
+            if (g) cudaGraphDestroy(g);
+            cudaGetLastError();
+            throw;
+        }
         const cudaError_t e1 = cudaGetLastError();
         const cudaError_t e2 = cudaStreamEndCapture(st_, &g);
         if (e1 != cudaSuccess || e2 != cudaSuccess) {

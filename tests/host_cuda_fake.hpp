@@ -64,7 +64,7 @@ cudaError_t cudaMallocFromPoolAsync(void** p, size_t n, cudaMemPool_t, cudaStrea
     return cudaSuccess;
 }
 cudaError_t cudaFreeAsync(void* p, cudaStream_t) { FAKE(cudaFreeAsync); return fake::drop(fake::device, p); }
-cudaError_t cudaMallocHost(void** p, size_t n) { FAKE(cudaMallocHost); *p = std::malloc(n); return cudaSuccess; }
+cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { FAKE(cudaHostAlloc); *p = std::malloc(n); return cudaSuccess; }
 cudaError_t cudaFreeHost(void* p) { FAKE(cudaFreeHost); std::free(p); return cudaSuccess; }
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) {
     FAKE(cudaMemcpyAsync);
@@ -79,5 +79,40 @@ cudaError_t cudaMemPoolCreate(cudaMemPool_t* p, const cudaMemPoolProps*) {
 cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void*) { FAKE(cudaMemPoolSetAttribute); return cudaSuccess; }
 cudaError_t cudaMemPoolTrimTo(cudaMemPool_t, size_t) { FAKE(cudaMemPoolTrimTo); return cudaSuccess; }
 cudaError_t cudaGetSymbolAddress(void** p, const void* sym) { FAKE(cudaGetSymbolAddress); *p = const_cast<void*>(sym); return cudaSuccess; }
+cudaError_t cudaStreamGetPriority(cudaStream_t, int* p) { FAKE(cudaStreamGetPriority); *p = 0; return cudaSuccess; }
+cudaError_t cudaStreamCreateWithPriority(cudaStream_t* s, unsigned, int) {
+    FAKE(cudaStreamCreateWithPriority);
+    *s = (cudaStream_t)fake::make(fake::streams);
+    return cudaSuccess;
+}
+cudaError_t cudaStreamDestroy(cudaStream_t s) { FAKE(cudaStreamDestroy); return fake::drop(fake::streams, s); }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) {
+    FAKE(cudaEventCreateWithFlags);
+    *e = (cudaEvent_t)fake::make(fake::events);
+    return cudaSuccess;
+}
+cudaError_t cudaEventDestroy(cudaEvent_t e) { FAKE(cudaEventDestroy); return fake::drop(fake::events, e); }
+cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { FAKE(cudaEventRecord); return cudaSuccess; }
+cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { FAKE(cudaStreamWaitEvent); return cudaSuccess; }
+cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) {
+    FAKE(cudaStreamBeginCapture);
+    if (fake::capturing) return cudaErrorIllegalState;
+    fake::capturing = 1;
+    return cudaSuccess;
+}
+cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t* g) {
+    FAKE(cudaStreamEndCapture);
+    *g = (cudaGraph_t)fake::make(fake::device);
+    fake::capturing = 0;
+    return cudaSuccess;
+}
+cudaError_t cudaGraphDestroy(cudaGraph_t g) { FAKE(cudaGraphDestroy); return fake::drop(fake::device, g); }
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t* x, cudaGraph_t, unsigned long long) {
+    FAKE(cudaGraphInstantiate);
+    *x = (cudaGraphExec_t)fake::make(fake::device);
+    return cudaSuccess;
+}
+cudaError_t cudaGraphExecDestroy(cudaGraphExec_t x) { FAKE(cudaGraphExecDestroy); return fake::drop(fake::device, x); }
+cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { FAKE(cudaGraphLaunch); return fake::capturing ? cudaErrorIllegalState : cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { FAKE(cudaStreamSynchronize); return cudaSuccess; }
 }
