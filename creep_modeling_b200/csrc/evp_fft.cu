@@ -978,6 +978,9 @@ struct TuneKey {
     }
 };
 enum : int { TUNE_XFWD = 0, TUNE_Y = 1, TUNE_ZGREEN = 2 };
+// Written behind each line of the cache file: the kernels and radix sets that its tile was timed on.  Lines
+// of another generation are ignored, so their grids are timed again.
+static const char* const kTileGeneration = "g2";
 static std::mutex g_tune_m;
 static std::map<TuneKey, int> g_tuned;
 static std::string g_tune_path;
@@ -994,12 +997,13 @@ void fft_tune_cache(const std::string& path) {
     if (path.empty()) return;
     std::ifstream f(path);
     std::string line;
-    while (std::getline(f, line)) {  // "evp-tile pass rs ct n1 n2 n3 tile"
+    while (std::getline(f, line)) {  // "evp-tile pass rs ct n1 n2 n3 tile generation"
         std::istringstream is(line);
-        std::string tag;
+        std::string tag, gen;
         TuneKey k{};
         int t = 0;
-        if ((is >> tag >> k.pass >> k.rs >> k.ct >> k.n1 >> k.n2 >> k.n3 >> t) && tag == "evp-tile" && t > 0) g_tuned[k] = t;
+        if ((is >> tag >> k.pass >> k.rs >> k.ct >> k.n1 >> k.n2 >> k.n3 >> t >> gen) && tag == "evp-tile" && gen == kTileGeneration && t > 0)
+            g_tuned[k] = t;
     }
 }
 
@@ -1254,7 +1258,7 @@ int fft_autotune(const Dev& d, const FftPlan1D& pl1, const FftPlan1D& pl2, const
         const TuneKey& k = kv.first;
         if (f.is_open())
             f << "evp-tile " << k.pass << ' ' << k.rs << ' ' << k.ct << ' ' << k.n1 << ' ' << k.n2 << ' ' << k.n3 << ' '
-              << kv.second << '\n';
+              << kv.second << ' ' << kTileGeneration << '\n';
     }
     return (int)found.size();
 }
