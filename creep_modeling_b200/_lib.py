@@ -10,7 +10,7 @@ from pathlib import Path
 LIB_PATH = Path(__file__).resolve().parent / "_build" / "libevp_b200.so"
 
 EXPORTED = (
-    "evp_solve_file", "evp_open", "evp_advance", "evp_get_field", "evp_last_rows", "evp_stats", "evp_close",
+    "evp_solve_file", "evp_open", "evp_advance", "evp_get_field", "evp_field_size", "evp_last_rows", "evp_stats", "evp_close",
     "evp_kernel_times", "evp_green_apply", "evp_green_apply_noalloc", "evp_last_error", "evp_version",
     "evp_server_open", "evp_submit", "evp_submit_deadline", "evp_poll", "evp_wait", "evp_server_close",
     "evp_set_deadline", "evp_kernel_launches", "evp_newton_stats",
@@ -90,6 +90,8 @@ def load(path: Path | str | None = None):
     L.evp_advance.restype = ctypes.c_int
     L.evp_get_field.argtypes = [vp, ctypes.c_char_p, c_dp, ctypes.c_longlong, ctypes.POINTER(ctypes.c_longlong)]
     L.evp_get_field.restype = ctypes.c_int
+    L.evp_field_size.argtypes = [vp, ctypes.c_char_p, ctypes.POINTER(ctypes.c_longlong)]
+    L.evp_field_size.restype = ctypes.c_int
     L.evp_last_rows.argtypes = [vp, c_dp, c_dp]
     L.evp_last_rows.restype = ctypes.c_int
     L.evp_stats.argtypes = [vp, ctypes.POINTER(Report)]

@@ -1422,14 +1422,14 @@ public:
         for (cudaError_t e : rc) CK(e);
     }
 
-    // Doubles written; -2: no such field; -16 - n: the buffer is too small for the field's n doubles.
+    // Doubles written (out null: the field's length); -1: the buffer is too small; -2: no such field.
     long long get_field(const std::string& name, double* out, long long cap) {
         const long long N = d.N;
         const int ns = d.nsys;
         auto soa_to_aos = [&](double* dp, const int* map, int nout) -> long long {
             const long long total = (long long)nout * N;
-            if (total > cap) return -total - 16;
-            if (total == 0) return 0;
+            if (!out || total == 0) return total;
+            if (total > cap) return -1;
             // interleaved on the device, in the spectrum's memory (free between increments), then copied
             const long long room = 2 * (long long)spec_size / nout;
             for (long long v0 = 0; v0 < N; v0 += room) {
@@ -1468,7 +1468,8 @@ public:
         if (name == "c066mod") return soa_to_aos(d.c066mod, m.data(), 36);
         if (name == "sg66") return soa_to_aos(d.sg66, m.data(), 36);
         if (name == "macro") {  // c066, c0, s0, de_ds (reference-medium state, host copies)
-            if (cap < 279) return -279 - 16;
+            if (!out) return 279;
+            if (cap < 279) return -1;
             std::memcpy(out, c066, sizeof(c066));
             std::memcpy(out + 36, c0, sizeof(c0));
             std::memcpy(out + 117, s0, sizeof(s0));
@@ -1477,7 +1478,8 @@ public:
         }
         if (name == "xnode") {
             long long n = 3LL * (d.n1 + 1) * (d.n2 + 1) * d.n3node;
-            if (n > cap) return -n - 16;
+            if (!out) return n;
+            if (n > cap) return -1;
             to_host(out, d.xnode, (size_t)n);
             return n;
         }
@@ -1801,14 +1803,23 @@ int evp_get_field(evp_solve* h, const char* name, double* host_out, long long ca
     try {
         long long n = h->s.get_field(name, host_out, capacity);
         if (n == -2) return fail(std::string("evp_get_field: unknown field ") + name, -7);
-        if (n < 0) {
-            if (written) *written = -n - 16;
-            return fail("evp_get_field: buffer too small", -7);
-        }
+        if (n < 0) return fail("evp_get_field: buffer too small", -7);
         if (written) *written = n;
     } catch (SolveError& e) {
         return fail(e.what(), e.code);
     } catch (std::exception& e) {  // a copying thread that could not start
+        return fail(e.what(), -6);
+    }
+    return 0;
+}
+
+int evp_field_size(evp_solve* h, const char* name, long long* size) {
+    if (!h || !name || !size) return fail("evp_field_size: null argument", -7);
+    try {
+        const long long n = h->s.get_field(name, nullptr, 0);
+        if (n < 0) return fail(std::string("evp_field_size: unknown field ") + name, -7);
+        *size = n;
+    } catch (std::exception& e) {
         return fail(e.what(), -6);
     }
     return 0;

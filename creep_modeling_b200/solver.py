@@ -88,16 +88,11 @@ class Solve:
         return r, d
 
     def field(self, name: str) -> np.ndarray:
-        lib, n, one = _lib.load(), ctypes.c_longlong(-1), np.empty(1)
-        dp = ctypes.POINTER(ctypes.c_double)
-        # a buffer of one value: the call says how many the field has (or that it has none of that name)
-        rc = lib.evp_get_field(self._h, name.encode(), one.ctypes.data_as(dp), 1, ctypes.byref(n))
-        if rc == 0:
-            return one[: n.value]
-        if n.value < 0:
-            _lib.check(rc)
+        lib, n = _lib.load(), ctypes.c_longlong(0)
+        _lib.check(lib.evp_field_size(self._h, name.encode(), ctypes.byref(n)))
         buf = np.empty(n.value)
-        _lib.check(lib.evp_get_field(self._h, name.encode(), buf.ctypes.data_as(dp), buf.size, ctypes.byref(n)))
+        _lib.check(lib.evp_get_field(self._h, name.encode(), buf.ctypes.data_as(ctypes.POINTER(ctypes.c_double)), buf.size,
+                                     ctypes.byref(n)))
         return buf
 
     def kernel_times(self) -> dict:

@@ -74,8 +74,9 @@ int evp_advance(evp_solve* s, int nmacro, int* done);
  * velgradold, defgrad, defgradinv, defgrade, defgradp, edotp, ept,
  * disgradsym, dvelgradref, gamdot, crss, trialtau, sch, c066mod, sg66, detF,
  * wgtc, gacumgr, epvm, xnode.  *written = number of doubles copied; a buffer that
- * is too small is refused (-7) and *written says how many the field has. */
+ * is too small is refused (-7).  evp_field_size: the number of doubles that a field has. */
 int evp_get_field(evp_solve* s, const char* name, double* host_out, long long capacity, long long* written);
+int evp_field_size(evp_solve* s, const char* name, long long* size);
 
 /* Last results.csv row (51 values, IO_functions.f90:1264-1271 order) and
  * diagnostics.csv row (44 values, types.f90:787-798 order). */
