@@ -14,12 +14,15 @@ namespace evp {
         if (e_ != cudaSuccess) throw SolveError(std::string("CUDA error: ") + cudaGetErrorString(e_), -6); \
     } while (0)
 
-cudaMemPool_t solver_pool() {
+// The pools of each device: [0] the solves', [1] the bare operator's.  Made at their first use.
+static std::mutex g_pool_m;
+static std::map<int, cudaMemPool_t> g_pools[2];
+
+static cudaMemPool_t pool_of(int which, unsigned long long keep) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) throw SolveError("cudaGetDevice failed", -6);
-    static std::mutex m;
-    static std::map<int, cudaMemPool_t> pools;
-    std::lock_guard<std::mutex> lk(m);
+    std::lock_guard<std::mutex> lk(g_pool_m);
+    auto& pools = g_pools[which];
     auto it = pools.find(dev);
     if (it != pools.end()) return it->second;
     cudaMemPoolProps props{};
@@ -29,10 +32,20 @@ cudaMemPool_t solver_pool() {
     props.location.id = dev;
     cudaMemPool_t pool;
     ECK(cudaMemPoolCreate(&pool, &props));
-    unsigned long long keep = ~0ull;
     ECK(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
     pools.emplace(dev, pool);
     return pool;
+}
+cudaMemPool_t solver_pool() { return pool_of(0, ~0ull); }
+cudaMemPool_t operator_pool() { return pool_of(1, kOperatorPoolKeep); }
+void release_pools() {
+    int dev = 0;
+    ECK(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lk(g_pool_m);
+    for (auto& pools : g_pools) {
+        auto it = pools.find(dev);
+        if (it != pools.end()) ECK(cudaMemPoolTrimTo(it->second, 0));
+    }
 }
 
 static const char* kind_name(int k) {

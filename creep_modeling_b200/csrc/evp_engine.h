@@ -30,6 +30,11 @@ struct SolveError : std::runtime_error {
 // The library's device memory pool of the current device (stream-ordered allocations that
 // stay with the process instead of going back to the driver at every synchronisation).
 cudaMemPool_t solver_pool();
+// The pool of the bare operator's scratch, which keeps at most this much between calls.
+constexpr unsigned long long kOperatorPoolKeep = 256ull << 20;
+cudaMemPool_t operator_pool();
+// Gives what no allocation uses in the current device's pools back to the driver.
+void release_pools();
 
 class Engine {
 public:

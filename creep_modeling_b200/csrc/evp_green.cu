@@ -97,18 +97,17 @@ extern "C" int evp_green_apply(const double* d_tau, double* d_out, int n1, int n
     d.n1h = n1 / 2 + 1;
     d.N = (long long)n1 * n2 * n3;
     // Scratch: the half spectrum, then what the host supplies (twiddles, c0 and s0, the error word) as
-    // one upload.  From the library's pool up to kPoolMost, where a fresh allocation and its release
-    // cost more than the transforms (64^3: 0.86 ms a call before, 0.17 now; 120x90x80: 2.5 and 0.58); a
-    // larger one is given back to the device.
-    constexpr size_t kPoolMost = (size_t)1 << 30;
+    // one upload.  From a pool of its own up to what that keeps between calls (a 128^3 grid: 153 MB), where a
+    // fresh allocation and its release cost more than the transforms (64^3: 0.86 ms a call before, 0.17 now;
+    // 120x90x80: 2.5 and 0.58); a larger one is given back to the device.
     const size_t nspec = 9 * (size_t)d.n1h * n2 * n3, ntw = (size_t)n1 + n2 + n3, ntail = ntw + 81 + 1;
     const size_t bytes = (nspec + ntail) * sizeof(double2);
     std::vector<double2> tail;
-    const bool pooled = bytes <= kPoolMost;
+    const bool pooled = bytes <= kOperatorPoolKeep;
     void* mem = nullptr;
     try {
         tail.resize(ntail);
-        const cudaError_t ae = pooled ? cudaMallocFromPoolAsync(&mem, bytes, solver_pool(), st) : cudaMalloc(&mem, bytes);
+        const cudaError_t ae = pooled ? cudaMallocFromPoolAsync(&mem, bytes, operator_pool(), st) : cudaMalloc(&mem, bytes);
         if (ae != cudaSuccess) {
             cudaGetLastError();
             set_last_error("evp_green_apply: device allocation failed");
@@ -132,6 +131,16 @@ extern "C" int evp_green_apply(const double* d_tau, double* d_out, int n1, int n
     if (pooled) cudaFreeAsync(mem, st);
     else cudaFree(mem);
     return rc;
+}
+
+extern "C" int evp_release_memory(void) {
+    try {
+        evp::release_pools();
+    } catch (std::exception& e) {
+        evp::set_last_error(e.what());
+        return -6;
+    }
+    return 0;
 }
 
 // ---------------------------------------------------------------- allocation-free variant

@@ -110,10 +110,14 @@ int evp_newton_stats(evp_solve* s, long long* out6);
  * outermost (field[c*N + v], v = i + n1*(j + n2*k)); d_out may not alias d_tau.
  * c0, s0: host arrays of 81 doubles, the reference stiffness and its
  * compliance (4th-order, index ((i*3+j)*3+k)*3+l).  stream: a cudaStream_t or
- * NULL.  The scratch spectrum is taken inside the call (up to 1 GB from the library's memory pool, which
- * keeps it for later calls and solves; above that allocated and freed). */
+ * NULL.  The scratch spectrum is taken inside the call: up to 256 MB from a memory pool, which keeps that
+ * much for later calls (evp_release_memory gives it back); a larger one is allocated and freed. */
 int evp_green_apply(const double* d_tau, double* d_out, int n1, int n2, int n3, const double* c0, const double* s0,
                     void* stream);
+
+/* Give the device memory that the library keeps on the current device for later solves and operator calls,
+ * and that none is using, back to the driver. */
+int evp_release_memory(void);
 
 /* Allocation-free variant of evp_green_apply (no counterpart in the reference,
  * whose Fortran solver has no device and no allocator to avoid).  For callers
