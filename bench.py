@@ -56,7 +56,7 @@ def algorithmic_bytes(n1: int, nsys: int = 12) -> dict:
     }
 
 
-# Counted FP64 arithmetic of k_newtonv (12 slip systems; a fused multiply-add counts 2, the integer
+# Counted FP64 arithmetic of k_newton (12 slip systems; a fused multiply-add counts 2, the integer
 # power |x|^(n-1) by binary powering 8): one constitutive evaluation (resolved shears, power law,
 # plastic strain rate, tangent dd, residual rho and C~ rho, their norm) 970; one Newton step (H, its
 # L D L^T factors, the substitutions, the update and its norm) 190; one hardening update (the slip

@@ -14,6 +14,7 @@
 namespace evp {
 
 constexpr int kMaxSysDev = 24;
+constexpr int kMaxPhaseSmem = 3;  // phases whose tables the local solve keeps in shared memory
 
 // Per-phase constants (phase_type, types.f90:96-118) in device memory.
 struct PhaseDev {
@@ -203,7 +204,7 @@ struct Job {
 // iteration of an increment starts from is formed when the increment's iterations start).
 enum BatchKind : int { BK_XFWD, BK_YFWD, BK_ZGREEN, BK_YINV, BK_XINV, BK_CORR, BK_NEWTON, BK_N };
 struct BatchLaunch {
-    int kind, variant;  // variant: FFT passes rs | (FP32 << 2); Newton: the kernel (newton_variant)
+    int kind, variant;  // variant: FFT passes rs | (FP32 << 2); Newton: newton_shape()
     int job0, njobs;    // slice of the plan's job table
     int blocks, threads;
     size_t smem;
@@ -262,8 +263,6 @@ void launch_goperr0(const Dev& d, const double* c0, const double* s0, int igamma
 // form_G for IGAMMA 1 and 2: tabulate the Green operator at every half-spectrum point
 void launch_goper_tab(const Dev& d, const double* c0, const double* s0, int igamma, cudaStream_t st);
 void launch_gas_compl(const Dev& d, double tdot, double complgas, int modal, cudaStream_t st);
-void launch_corr(const Dev& d, const CorrParams& p, cudaStream_t st);
-void launch_newton(const Dev& d, const NewtonParams& p, cudaStream_t st);
 void launch_upd1(const Dev& d, const Upd1Params& p, cudaStream_t st);
 void launch_upd2(const Dev& d, const Upd2Params& p, cudaStream_t st);
 void launch_upd3(const Dev& d, const Upd3Params& p, cudaStream_t st);

@@ -393,16 +393,6 @@ __device__ __forceinline__ void body_corr(const Dev& d, const CorrParams& p, con
     }
     reduce_store<31, 0>(s, nullptr, d.partials, d.red + OFF_CORR, d.counters + CNT_CORR, vb);
 }
-__global__ void __launch_bounds__(kBlock, 2) k_corr(Dev d, CorrParams p) {
-    if (d.cgas) body_corr<true>(d, p, hw_vb());
-    else body_corr<false>(d, p, hw_vb());
-}
-// fewer blocks than the other voxel kernels: each thread handles several voxels, which spreads the
-// 31-field block reduction over more loads
-void launch_corr(const Dev& d, const CorrParams& p, cudaStream_t st) {
-    const int grid = d.grid < 148 * 2 ? d.grid : 148 * 2;
-    k_corr<<<grid, d.block, 0, st>>>(d, p);
-}
 
 // ---------------------------------------------------------------- batched launches of the iteration's voxel passes
 // Each block finds its member in the launch's parameter (binary search on blk0), reads
@@ -430,7 +420,9 @@ void member_jobs_voxel(const Dev& d, MemberJobs& mj) {
         mj.smem[0][k] = sm;
         mj.variant[0][k] = variant;
     };
-    // members of one block size share a launch: variant = (no gas phase) + 2 * (block size / 32)
+    // k_corr: fewer blocks than the other voxel kernels, so that each thread's several voxels spread the
+    // 31-field block reduction over more loads; members of one block size share a launch:
+    // variant = (no gas phase) + 2 * (block size / 32)
     one_d(BK_CORR, d.grid < 148 * 2 ? d.grid : 148 * 2, d.block, 0, (d.cgas ? 0 : 1) + 2 * (d.block / 32));
     const NewtonShape n = newton_shape(d);
     one_d(BK_NEWTON, n.grid, n.threads, n.smem, n.variant);

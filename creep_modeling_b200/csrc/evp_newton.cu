@@ -5,217 +5,11 @@
 #include "evp_math.cuh"
 #include "evp_vox.cuh"
 
-#include <cstdlib>
 #include <mutex>
 
 namespace evp {
 
-// ---------------------------------------------------------------- k_newton
-template <int NS>
-__device__ __forceinline__ void body_newton1(const Dev& d, const NewtonParams& p, const VB& vb) {
-    const long long N = d.N;
-    double s[14];
-#pragma unroll
-    for (int c = 0; c < 14; c++) s[c] = 0.0;
-    for (long long v = vb.x * (long long)blockDim.x + threadIdx.x; v < N; v += (long long)vb.nx * blockDim.x) {
-        double lam[6], sg[6], sgt[6], D[6];
-        {
-            double vg[9], vs[9], a[6];
-            ld9(d.velgrad, N, v, vg);
-            sym33(vg, vs);
-            t2_to_b6(vs, D);
-            ld6(d.sg, N, v, a);
-            s6_to_b6(a, lam);
-            ld6(d.sgt, N, v, a);
-            s6_to_b6(a, sgt);
-        }
-#pragma unroll
-        for (int i = 0; i < 6; i++) sg[i] = lam[i];
-        const double w = d.wgtc[v];
-        if (d.gas[v]) {
-            double t[6], res[6], out[6], s6v[6];
-#pragma unroll
-            for (int i = 0; i < 6; i++) t[i] = D[i] + sgt[i] / p.tdot * p.complgas;
-#pragma unroll
-            for (int i = 0; i < 6; i++) {
-                double a = 0.0;
-#pragma unroll
-                for (int j = 0; j < 6; j++) a += d.c066mod[(6 * i + j) * N + v] * t[j];
-                res[i] = lam[i] + a;
-            }
-            if (p.modal) {
-#pragma unroll
-                for (int i = 0; i < 6; i++) {
-                    double a = 0.0;
-#pragma unroll
-                    for (int j = 0; j < 6; j++) a += d.cG[(6 * i + j) * N + v] * lam[j];
-                    res[i] -= a;
-                }
-            }
-#pragma unroll
-            for (int i = 0; i < 6; i++) {
-                double a = 0.0;
-#pragma unroll
-                for (int j = 0; j < 6; j++) a += d.cgas[(6 * i + j) * N + v] * res[j];
-                out[i] = a;
-            }
-            b6_to_s6(out, s6v);
-            st6(d.sg, N, v, s6v);
-            double z[6] = {0, 0, 0, 0, 0, 0};
-            st6(d.edotp, N, v, z);
-            for (int q = 0; q < d.nsys; q++) d.gamdot[q * N + v] = 0.0;
-#pragma unroll
-            for (int c = 0; c < 6; c++) s[8 + c] += s6v[c] * w;
-            continue;
-        }
-        const PhaseDev& ph = d.ph[d.phase[v]];
-        double tt[NS][2];
-        double taunrm = 0.0;
-#pragma unroll
-        for (int q = 0; q < NS; q++) {
-            tt[q][0] = (q < d.nsys) ? d.trialtau[(2 * q) * N + v] : 0.0;
-            tt[q][1] = (q < d.nsys) ? d.trialtau[(2 * q + 1) * N + v] : 0.0;
-            taunrm += tt[q][0] * tt[q][0] + tt[q][1] * tt[q][1];
-        }
-        taunrm = sqrt(taunrm);
-        double edotth[6] = {0, 0, 0, 0, 0, 0};
-        if (p.thermo) {
-            double e9[9];
-            ld9(d.eth, N, v, e9);
-            t2_to_b6(e9, edotth);
-        }
-        double sgnorm = 0.0;
-#pragma unroll
-        for (int i = 0; i < 6; i++) sgnorm += sg[i] * sg[i];
-        sgnorm = sqrt(sgnorm);
-        const double tolt = fmax(p.error, p.erroral);
-        double errtau = 2.0 * tolt;
-        double edotp[6], dd[15], gamdot[NS], edot[6], res[6], sgold[6] = {0, 0, 0, 0, 0, 0};
-        double dsgnorm = 0.0, ddgnorm = 0.0;
-        const double gamma0 = d.gacumgr[v];
-        for (int itertau = 0; itertau < 10 && errtau > tolt;) {
-            itertau++;
-            int iterNR = 0;
-            double erral = 2.0 * p.erroral, resoldn = 1.0;
-            while (iterNR < 100 && erral > p.erroral) {
-                iterNR++;
-                int icut = 0;
-                double resn = 2.0 * resoldn;
-                while (resn > resoldn && icut < 10) {
-                    constitutive<NS>(ph, d.sch, N, v, tt, sg, edotp, dd, gamdot);
-                    double ds[6];
-#pragma unroll
-                    for (int i = 0; i < 6; i++) ds[i] = (sg[i] - sgt[i]) / p.tdot;
-#pragma unroll
-                    for (int i = 0; i < 6; i++) {
-                        double a = 0.0;
-#pragma unroll
-                        for (int j = 0; j < 6; j++) a += d.sg66[(6 * i + j) * N + v] * ds[j];
-                        edot[i] = edotp[i] + a;
-                        if (p.thermo) edot[i] = edot[i] + edotth[i];
-                    }
-#pragma unroll
-                    for (int i = 0; i < 6; i++) {
-                        double a = 0.0;
-#pragma unroll
-                        for (int j = 0; j < 6; j++) a += d.c066mod[(6 * i + j) * N + v] * (edot[j] - D[j]);
-                        res[i] = sg[i] - lam[i] + a;
-                    }
-                    if (p.modal) {
-                        double r2[6];
-#pragma unroll
-                        for (int i = 0; i < 6; i++) {
-                            double a = 0.0;
-#pragma unroll
-                            for (int j = 0; j < 6; j++) a += d.cG[(6 * i + j) * N + v] * (sg[j] - lam[j]);
-                            r2[i] = a;
-                        }
-#pragma unroll
-                        for (int i = 0; i < 6; i++) res[i] = res[i] - r2[i];
-                    }
-                    resn = 0.0;
-#pragma unroll
-                    for (int i = 0; i < 6; i++) resn += res[i] * res[i];
-                    resn = sqrt(resn);
-                    if (iterNR == 1) resoldn = resn;
-                    if (resn > resoldn) {
-#pragma unroll
-                        for (int i = 0; i < 6; i++) sg[i] = sgold[i] + (sg[i] - sgold[i]) * 0.5;
-                    }
-                    icut++;
-                }
-                resoldn = resn;
-#pragma unroll
-                for (int i = 0; i < 6; i++) sgold[i] = sg[i];
-                double J[36];
-#pragma unroll
-                for (int i = 0; i < 6; i++) {
-                    double crow[6];
-#pragma unroll
-                    for (int k = 0; k < 6; k++) crow[k] = d.c066mod[(6 * i + k) * N + v];
-#pragma unroll
-                    for (int j = 0; j < 6; j++) {
-                        double a = 0.0;
-#pragma unroll
-                        for (int k = 0; k < 6; k++) a += crow[k] * (dd_at(dd, k, j) + d.sg66[(6 * k + j) * N + v] / p.tdot);
-                        J[6 * i + j] = ((i == j) ? 1.0 : 0.0) + a;
-                        if (p.modal) J[6 * i + j] -= d.cG[(6 * i + j) * N + v];
-                    }
-                }
-                if (solve6(J, res) != 0) set_err(d.err, 1);
-                double a = 0.0, b = 0.0, c = 0.0;
-#pragma unroll
-                for (int i = 0; i < 6; i++) {
-                    sg[i] = sg[i] - res[i];
-                    a += (sg[i] - sgold[i]) * (sg[i] - sgold[i]);
-                    b += (sg[i] - lam[i]) * (sg[i] - lam[i]);
-                    c += (edot[i] - D[i]) * (edot[i] - D[i]);
-                }
-                dsgnorm = b;
-                ddgnorm = c;
-                erral = sqrt(a) / sgnorm;
-            }
-            if (p.iuphard) {
-                double tn[NS][2], g1;
-                harden<NS>(ph, d.crss, N, v, gamdot, gamma0, p.tdot, tn, g1);
-                double e2 = 0.0;
-#pragma unroll
-                for (int q = 0; q < NS; q++) {
-                    e2 += (tt[q][0] - tn[q][0]) * (tt[q][0] - tn[q][0]) + (tt[q][1] - tn[q][1]) * (tt[q][1] - tn[q][1]);
-                    tt[q][0] = tn[q][0];
-                    tt[q][1] = tn[q][1];
-                }
-                errtau = sqrt(e2) / taunrm;
-            } else {
-                errtau = 0.0;
-            }
-        }
-        double s6v[6], e6v[6];
-        b6_to_s6(sg, s6v);
-        b6_to_s6(edotp, e6v);
-        st6(d.sg, N, v, s6v);
-        st6(d.edotp, N, v, e6v);
-#pragma unroll
-        for (int q = 0; q < NS; q++)
-            if (q < d.nsys) {
-                d.gamdot[q * N + v] = gamdot[q];
-                d.trialtau[(2 * q) * N + v] = tt[q][0];
-                d.trialtau[(2 * q + 1) * N + v] = tt[q][1];
-            }
-        if (!(dsgnorm == dsgnorm) || !(ddgnorm == ddgnorm)) set_err(d.err, 2);
-        s[0] += dsgnorm * w;
-        s[1] += ddgnorm * w;
-#pragma unroll
-        for (int c = 0; c < 6; c++) {
-            s[2 + c] += w * s6v[c];
-            s[8 + c] += s6v[c] * w;
-        }
-    }
-    reduce_store<14, 0>(s, nullptr, d.partials, d.red + OFF_NEWTON, d.counters + CNT_NEWTON, vb);
-}
-template <int NS>
-__global__ void __launch_bounds__(kNewtonBlock, 2) k_newton(Dev d, NewtonParams p) { body_newton1<NS>(d, p, hw_vb()); }
-// ---------------------------------------------------------------- k_newtonv: one voxel per thread, operators on chip
+// ---------------------------------------------------------------- k_newton: one voxel per thread, operators on chip
 // The local solve with one thread per voxel and everything an evaluation reads kept in the
 // block's shared memory, one column per thread (entry i of thread t at [i * blockDim + t], so
 // every access of a warp is conflict free).  With dedot = dd + S / dt the Jacobian of solve_res is
@@ -248,7 +42,6 @@ __global__ void __launch_bounds__(kNewtonBlock, 2) k_newton(Dev d, NewtonParams 
 // too; every operator is taken with its 36 entries and H goes to the pivoted elimination.  The wider column
 // leaves room for 128 threads per SM: 485 us at 64^3 (630 with six lanes per voxel, 1600 with every operator
 // re-read from memory), 231 at 40^3 with 24 systems (365), 42 at 16^3 (36).
-constexpr int kMaxPhaseSmem = 4;
 // column entries of a thread: Schmid vectors, 1 / resistance (forward, backward), H0 (packed lower triangle, or all of it)
 template <int NS, bool SYM>
 struct ColV {
@@ -481,7 +274,7 @@ __device__ __forceinline__ void body_newtonv(const Dev& d, const NewtonParams& p
     using Op = Op6<SYM>;
     extern __shared__ __align__(16) double dyn_smem[];
     PhaseV<NS>* const sph = reinterpret_cast<PhaseV<NS>*>(dyn_smem);
-    const int nph = d.nph;  // at most kMaxPhaseSmem (newton_kernel)
+    const int nph = d.nph;  // at most kMaxPhaseSmem
     for (int e = threadIdx.x; e < nph * (int)(sizeof(PhaseV<NS>) / 8); e += blockDim.x) dyn_smem[e] = d.phv[e];
     __syncthreads();
     const int lane = threadIdx.x & 31;
@@ -833,81 +626,52 @@ __device__ __forceinline__ void body_newtonv(const Dev& d, const NewtonParams& p
     }
     reduce_newton(sh, d.partials, d.red + OFF_NEWTON, d.counters + CNT_NEWTON, vb);
 }
-template <int NS, bool UNI, bool SYM>
-__global__ void __launch_bounds__(newtonv_threads_per_sm<NS, SYM>(), 1) k_newtonv(Dev d, NewtonParams p) { body_newtonv<NS, UNI, SYM>(d, p, hw_vb()); }
 
-// The local-solve kernel of a solve: 0/1 k_newtonv<12/24> for integer exponents, 2/3 for others, 4/5 for
-// any with a phase of asymmetric stiffness (at most kMaxPhaseSmem phases, whose tables fit beside the
-// columns), 6/7 k_newton<12/24>, which reads every operator from memory (more phases, and
-// EVP_NEWTON_ONE_THREAD=1 for comparison).
-static int newton_kernel(const Dev& d) {
-    static const bool one_thread = [] {
-        const char* e = getenv("EVP_NEWTON_ONE_THREAD");
-        return e && e[0] == '1';
-    }();
-    const int big = d.nsys > 12 ? 1 : 0;
-    return (one_thread || d.nph > kMaxPhaseSmem ? 6 : (!d.symel ? 4 : (d.uniexp ? 0 : 2))) + big;
-}
+// The local-solve kernel of a solve: 0/1 body_newtonv<12/24> for integer exponents, 2/3 for others, 4/5 for
+// any with a phase of asymmetric stiffness.
+static int newton_kernel(const Dev& d) { return (!d.symel ? 4 : (d.uniexp ? 0 : 2)) + (d.nsys > 12 ? 1 : 0); }
 constexpr int newton_sm_threads(int kernel) {
     return kernel >= 4 ? newtonv_threads_per_sm<12, false>() : (kernel & 1 ? newtonv_threads_per_sm<24, true>() : newtonv_threads_per_sm<12, true>());
 }
-// Block size of k_newtonv: as many threads as an SM holds (one block per SM, the fewest partial
+// Block size: as many threads as an SM holds (one block per SM, the fewest partial
 // sums to fold) unless that leaves SMs without a block; then halved until every SM has one, down
 // to one warp.
 static int newton_threads(const Dev& d, int kernel) {
-    if (kernel >= 6) return kNewtonBlock;
     int t = newton_sm_threads(kernel);
     while (t > 32 && (d.N + t - 1) / t < 148) t /= 2;
     return t;
 }
 static int newton_grid(const Dev& d, int kernel) {
     const long long t = newton_threads(d, kernel), g = (d.N + t - 1) / t;
-    if (kernel >= 6) return (int)(g < 148LL * 16 ? g : 148LL * 16);
     // one wave, every warp taking every (blocks x warps)-th batch of 32 voxels
     const long long wave = 148LL * (newton_sm_threads(kernel) / t);
     return (int)(g < wave ? g : wave);
 }
 static size_t newton_smem(const Dev& d, int kernel) {
     const size_t t = newton_threads(d, kernel);
-    if (kernel >= 6) return 0;
     const size_t entries = kernel >= 4 ? (kernel & 1 ? ColV<24, false>::n : ColV<12, false>::n) : (kernel & 1 ? ColV<24, true>::n : ColV<12, true>::n);
     return d.nph * (kernel & 1 ? sizeof(PhaseV<24>) : sizeof(PhaseV<12>)) + sizeof(double) * entries * t;
 }
+// dynamic shared memory that a block may take beside the kernel's own (the SM's limit of 227 KB less 5)
+constexpr int kNewtonSmemMost = 222 * 1024;
+static_assert(kMaxPhaseSmem * sizeof(PhaseV<12>) + sizeof(double) * ColV<12, true>::n * newtonv_threads_per_sm<12, true>() <= kNewtonSmemMost &&
+              kMaxPhaseSmem * sizeof(PhaseV<24>) + sizeof(double) * ColV<24, true>::n * newtonv_threads_per_sm<24, true>() <= kNewtonSmemMost &&
+              kMaxPhaseSmem * sizeof(PhaseV<12>) + sizeof(double) * ColV<12, false>::n * newtonv_threads_per_sm<12, false>() <= kNewtonSmemMost &&
+              kMaxPhaseSmem * sizeof(PhaseV<24>) + sizeof(double) * ColV<24, false>::n * newtonv_threads_per_sm<24, false>() <= kNewtonSmemMost,
+              "the phases' tables and the columns fit");
 template <int V>
-constexpr int kb_newton_bound() { return V >= 6 ? kNewtonBlock : newton_sm_threads(V); }
-template <int V>
-__global__ void __launch_bounds__(kb_newton_bound<V>(), V >= 6 ? 2 : 1) kb_newton(const __grid_constant__ BatchParams P);
+__global__ void __launch_bounds__(newton_sm_threads(V), 1) kb_newton(const __grid_constant__ BatchParams P);
 static void newton_configure() {
     static std::once_flag once;
     std::call_once(once, [] {
-        const int lim = 222 * 1024;
-        const void* const ks[] = {(const void*)k_newtonv<12, true, true>, (const void*)k_newtonv<24, true, true>,
-                                  (const void*)k_newtonv<12, false, true>, (const void*)k_newtonv<24, false, true>,
-                                  (const void*)k_newtonv<12, false, false>, (const void*)k_newtonv<24, false, false>,
-                                  (const void*)kb_newton<0>, (const void*)kb_newton<1>, (const void*)kb_newton<2>,
+        const void* const ks[] = {(const void*)kb_newton<0>, (const void*)kb_newton<1>, (const void*)kb_newton<2>,
                                   (const void*)kb_newton<3>, (const void*)kb_newton<4>, (const void*)kb_newton<5>};
-        for (const void* k : ks) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+        for (const void* k : ks) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kNewtonSmemMost);
     });
 }
 
-void launch_newton(const Dev& d, const NewtonParams& p, cudaStream_t st) {
-    newton_configure();
-    const int k = newton_kernel(d), grid = newton_grid(d, k), thr = newton_threads(d, k);
-    const size_t sm = newton_smem(d, k);
-    switch (k) {
-        case 0: k_newtonv<12, true, true><<<grid, thr, sm, st>>>(d, p); break;
-        case 1: k_newtonv<24, true, true><<<grid, thr, sm, st>>>(d, p); break;
-        case 2: k_newtonv<12, false, true><<<grid, thr, sm, st>>>(d, p); break;
-        case 3: k_newtonv<24, false, true><<<grid, thr, sm, st>>>(d, p); break;
-        case 4: k_newtonv<12, false, false><<<grid, thr, sm, st>>>(d, p); break;
-        case 5: k_newtonv<24, false, false><<<grid, thr, sm, st>>>(d, p); break;
-        case 6: k_newton<12><<<grid, thr, 0, st>>>(d, p); break;
-        default: k_newton<24><<<grid, thr, 0, st>>>(d, p); break;
-    }
-}
-
 template <int V>
-__global__ void __launch_bounds__(kb_newton_bound<V>(), V >= 6 ? 2 : 1) kb_newton(const __grid_constant__ BatchParams P) {
+__global__ void __launch_bounds__(newton_sm_threads(V), 1) kb_newton(const __grid_constant__ BatchParams P) {
     __shared__ NewtonParams ps;
     __shared__ int go;
     const Job& jb = batch_job(P);
@@ -925,9 +689,7 @@ __global__ void __launch_bounds__(kb_newton_bound<V>(), V >= 6 ? 2 : 1) kb_newto
     else if constexpr (V == 2) body_newtonv<12, false, true>(m.d, p, vb);
     else if constexpr (V == 3) body_newtonv<24, false, true>(m.d, p, vb);
     else if constexpr (V == 4) body_newtonv<12, false, false>(m.d, p, vb);
-    else if constexpr (V == 5) body_newtonv<24, false, false>(m.d, p, vb);
-    else if constexpr (V == 6) body_newton1<12>(m.d, p, vb);
-    else body_newton1<24>(m.d, p, vb);
+    else body_newtonv<24, false, false>(m.d, p, vb);
 }
 
 // Launch shape of a solve's local solve.  Members of one block size share a batched launch:
@@ -944,9 +706,7 @@ void launch_batched_newton(const BatchLaunch& L, const BatchParams& P, cudaStrea
         case 2: kb_newton<2><<<L.blocks, L.threads, L.smem, st>>>(P); break;
         case 3: kb_newton<3><<<L.blocks, L.threads, L.smem, st>>>(P); break;
         case 4: kb_newton<4><<<L.blocks, L.threads, L.smem, st>>>(P); break;
-        case 5: kb_newton<5><<<L.blocks, L.threads, L.smem, st>>>(P); break;
-        case 6: kb_newton<6><<<L.blocks, L.threads, L.smem, st>>>(P); break;
-        default: kb_newton<7><<<L.blocks, L.threads, L.smem, st>>>(P); break;
+        default: kb_newton<5><<<L.blocks, L.threads, L.smem, st>>>(P); break;
     }
 }
 

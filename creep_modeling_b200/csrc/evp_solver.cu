@@ -460,6 +460,7 @@ public:
             twiddles_f(dk.n1, d.tw1f); twiddles_f(dk.n2, d.tw2f); twiddles_f(dk.n3, d.tw3f);
         }
         // phases
+        static_assert(kMaxPhases <= kMaxPhaseSmem && kMaxSys <= kMaxSysDev, "the local solve holds every deck's phases");
         std::vector<PhaseDev> ph(dk.nph);
         d.symel = 1;
         for (int p = 0; p < dk.nph; p++) {

@@ -7,7 +7,6 @@
 namespace evp {
 
 constexpr int kBlock = 256;
-constexpr int kNewtonBlock = 128;
 constexpr int kC0Block = 64;
 
 // ---------------------------------------------------------------- reductions
