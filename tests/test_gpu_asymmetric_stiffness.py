@@ -2,10 +2,12 @@
 they stand, IO_functions.f90:640-720): every operator formed from it is then asymmetric and each step has
 to use all of its entries, against the oracle."""
 import dataclasses
+from pathlib import Path
 
+import numpy as np
 import pytest
 
-from creep_modeling_b200 import decks
+from creep_modeling_b200 import Solve, decks, solve_files
 from tests import parity
 
 pytestmark = pytest.mark.gpu
@@ -40,3 +42,22 @@ def test_asymmetric_stiffness_matches_oracle(tmp_path, n, slip, modal, gas, nrs)
         assert parity.field_rel_err(g, o, f) <= parity.RTOL, f
     g.close()
     o.close()
+
+
+def test_in_a_batch_as_alone(tmp_path):
+    """Beside symmetric members, whose launches it does not share."""
+    ffts, alone, outs = [], [], []
+    for i, n in enumerate((8, 16, 12)):
+        case = decks.case_c1(nsteps=2)
+        case.n, case.ngrains = n, 8
+        ffts.append(decks.write_case(case, tmp_path / f"d{i}"))
+        if i < 2:
+            (tmp_path / f"d{i}" / "cuel.sx").write_text(CUEL)
+        alone.append(tmp_path / f"alone{i}")
+        outs.append(str(tmp_path / f"batch{i}") + "/")
+        with Solve(ffts[i], out_dir=str(alone[i]) + "/", mix=1, modal=0, csv_only=True) as s:
+            s.run()
+    assert all(r.status == 0 for r in solve_files(ffts, outs, modal=0, csv_only=True))
+    for a, b in zip(alone, outs):
+        x, y = (np.delete(np.loadtxt(Path(d) / "results.csv", delimiter=",", skiprows=1, ndmin=2), 4, axis=1) for d in (a, b))
+        np.testing.assert_array_equal(x, y)
