@@ -1,12 +1,11 @@
 // evp_engine.h -- the equilibrium-iteration engine: one or many solves advanced by batched launches.
 //
 // Per equilibrium iteration (LS-EVPFFT.f90:233-359) the engine queues, for all its
-// members at once, one launch per pass of the iteration (stress average, the five
-// spectral passes, correction, local Newton) and per kernel variant those members
-// need (radix set, FP64 / FP32 spectrum, Newton kernel), then k_control, which does
-// every member's serial tail on the device.  Each member's blocks run the body of
-// its single-solve kernel on its own grid and tile, so a solve gives the same bits
-// alone and in a batch.  Without a per-kernel timer the iterations are captured
+// members at once, one launch per pass of the iteration (the five spectral passes,
+// correction, local solve) and per kernel variant those members need (radix set,
+// FP64 / FP32 spectrum, local-solve kernel, block size), then k_control, which does
+// every member's serial tail on the device.  Each member's blocks cover its own
+// grid with its own tile, so a solve gives the same bits alone and in a batch.  Without a per-kernel timer the iterations are captured
 // once in a CUDA graph and replayed; the host reads the members' event codes only
 // every few iterations.
 #pragma once
@@ -40,7 +39,6 @@ class Engine {
 public:
     struct Member {
         BatchSolve e;
-        int modal;  // modified augmented Lagrangian (selects the Newton kernel)
         int prec;   // 1: the member may run FP32 spectra (mixed precision)
     };
     using Timer = std::function<void(const char*, const std::function<void()>&)>;

@@ -12,8 +12,9 @@
 //   y: C2C inverse
 //   x: C2R + epilogue (dvelgradref, and the F^{-1}-weighted average that
 //      correction_to_current needs, various_functions.f90:1085-1101)
-// Each pass stages pencils in shared memory and runs a mixed-radix Stockham
-// FFT (radices 2,3,4,5,7,8,11,13) with twiddles from a per-axis table.
+// Each pass runs a mixed-radix Stockham FFT (radices 2,3,4,5,7,8,11,13) over pencils in shared memory with
+// twiddles from a per-axis table.  The x passes stage their pencils there (rows are packed and unpacked);
+// the first and last stages of y and the outer ends of z read and write global memory themselves.
 // The grid-update path (integrate_tensor2, various_functions.f90:359-429) reuses
 // the same passes with a different z operator.
 #include "evp_dev.cuh"
@@ -110,8 +111,9 @@ __device__ __forceinline__ double root_sin(int k) {  // k a compile-time constan
 }
 // DFT of odd length R, its outputs handed to out(q, value) a pair at a time: with t_k = v_k + v_(R-k)
 // and u_k = v_k - v_(R-k), outputs q and R - q are A -+ i B, A = v_0 + sum_k cos(2 pi k q / R) t_k,
-// B = sum_k sin(2 pi k q / R) u_k.  Half the products of the plain sum, and no second array of R
-// values (the plain sum kept 2 R and read its roots from memory: 2 kB of spills in every all-radix kernel).
+// B = sum_k sin(2 pi k q / R) u_k.  Half the products of the plain sum, and no second array of R values nor
+// roots read from memory.  Spills stored by the all-radix FP64 kernels: y 3.7 -> 2.8 kB, z 7.4 -> 5.5, x inverse
+// 3.7 -> 2.9; what remains is the in-place stages' (fft_maxb_r).
 template <int R, bool INV, class CT, class Out>
 __device__ __forceinline__ void dft_odd(CT (&v)[R], const Out& out) {
     using T = typename CxT<CT>::T;
@@ -238,9 +240,11 @@ __device__ __forceinline__ void fft_stage(CT* s, int ES, int P, int n, int Ns, c
 // the full set, 13.8 without them, event-timed).  Butterflies per thread fall with the radix so that
 // no stage holds more than 16 complex values per thread: two for every power-of-two
 // radix with RS = 0; four for radices 2-4, two for 5-8 and one for 11 and 13
-// otherwise.  Every kernel then fits 128 registers, two blocks of 256
-// threads per SM; the launchers size blocks for the stage that needs the most
-// threads (stage_threads).
+// otherwise.  Two blocks of 256 threads per SM leave a thread 128 registers, which a stage that is in place in
+// shared memory exceeds in FP64: it holds up to 16 complex values through its barrier, so these kernels
+// spill (bytes stored, FP64, sets 0 / 1 / 2: y 320 / 1312 / 2752, z with the Green operator 712 / 2728 / 5464,
+// x inverse 64 / 1212 / 2936; FP32 set 0 none, z 8).  The launchers size blocks for the stage that needs the
+// most threads (stage_threads).
 __host__ __device__ constexpr int fft_maxb_r(int rs, int R) { return rs == 0 ? 2 : (R <= 4 ? 4 : (R <= 8 ? 2 : 1)); }
 
 // An odd-radix stage as a function of its own (ODD_CALL in fft_run): its registers are

@@ -11,7 +11,7 @@ namespace evp {
 
 // ---------------------------------------------------------------- k_newton: one voxel per thread, operators on chip
 // The local solve with one thread per voxel and everything an evaluation reads kept in the
-// block's shared memory, one column per thread (entry i of thread t at [i * blockDim + t], so
+// block's shared memory, one column per thread (entry i of a lane at [32 i + lane] of its warp's columns, so
 // every access of a warp is conflict free).  With dedot = dd + S / dt the Jacobian of solve_res is
 //   J = I - C~ G + C~ (S / dt + dd) = C~ H,   H = B + S / dt + dd,   B = C~^-1 - G,
 // where G = Gamma~r is the modified augmented Lagrangian's operator (zero without --modal 1;
@@ -24,7 +24,8 @@ namespace evp {
 // sends the voxel to the pivoted elimination of the general system.
 // The resistances are used as reciprocals, formed where they change (at the start and at each
 // hardening update, 1.2 per voxel) instead of at each evaluation (3 per voxel); the resistances
-// themselves go to their output array at each update and are read back for the change's norm.
+// themselves go to their output array at each update, and the old ones, for the norm of the change, are the
+// reciprocals inverted.
 //
 // What bounds it: latency (global loads of the batch, FP64 chains) at 8 warps per SM: 255 registers
 // a thread and the 840 B column both allow 256 threads per SM with 12 systems, 128 with 24; the

@@ -416,7 +416,7 @@ public:
         d.dv3 = dalloc<double>(3 * N);
         d.Fini = dk.idispini > 0 ? dalloc<double>(9 * N) : nullptr;
         d.xnode = dalloc<double>(3 * (size_t)(dk.n1 + 1) * (dk.n2 + 1) * d.n3node);
-        // block partials: voxel kernels (<= 1184 blocks x 117 sums), Newton (<= 3552 x 14), and the
+        // block partials: voxel kernels (<= 1184 blocks x 117 sums), the local solve (<= 1184 x 14), and the
         // x inverse pass (one block per <= 1 pair of rows x 9 sums)
         d.partials = dalloc<double>(std::max<size_t>(200 * 2048, 9 * ((size_t)dk.n2 * dk.n3 / 2 + 1)));
         d.red = dalloc<double>(RED_OUT_SIZE);
@@ -1033,7 +1033,7 @@ public:
         if (!begin_increment()) return false;
         if (!solo) {
             solo.reset(new Engine(st));
-            solo->set_members({Engine::Member{entry(), modal ? 1 : 0, prec}});
+            solo->set_members({Engine::Member{entry(), prec}});
         } else {
             solo->update_entry(0, entry());
         }
@@ -1605,7 +1605,7 @@ public:
             if (slots[id].state != 0 || !slots[id].s) continue;
             members.push_back(id);
             Solver& s = *slots[id].s;
-            m.push_back(Engine::Member{s.entry(), s.modal ? 1 : 0, s.prec});
+            m.push_back(Engine::Member{s.entry(), s.prec});
         }
         eng->set_members(m);
         dirty = false;

@@ -139,8 +139,8 @@ int evp_green_apply_noalloc(const double* d_tau, double* d_out, int n1, int n2, 
  * callers run one solver process per solve and two or three at once, utils/run.py:169-196,
  * calibrate.py:1053-1057).
  *
- * Every equilibrium iteration of the batch is one launch per pass (stress average, the
- * five FFT passes with the Green operator, correction, local Newton; per kernel variant
+ * Every equilibrium iteration of the batch is one launch per pass (the five FFT
+ * passes with the Green operator, correction, local Newton; per kernel variant
  * and per 40 members) over all running members, whatever their grid sizes and material
  * parameters, followed by a device-side controller that does each member's serial tail
  * (averages, boundary-condition update, error norms, convergence and time-step rules)
